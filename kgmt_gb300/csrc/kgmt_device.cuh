@@ -247,6 +247,14 @@ __device__ __forceinline__ uint32_t grid_item(const GridView& g, uint32_t j)
     return j < kSmemGridItems ? g.items_s[j] : __ldg(g.items_g + j);
 }
 
+// A culling grid wholly in shared memory (function-level propagation).
+struct BlockGrid {
+    const uint16_t* start;
+    const uint16_t* items;
+};
+
+__device__ __forceinline__ uint32_t grid_item(const BlockGrid& g, uint32_t j) { return g.items[j]; }
+
 // Consecutive step boxes of a trajectory share an end point, so the grid cell
 // of each end point is computed once and carried into the next step.  Since
 // grid_cell is monotone, the cell range of a step box [min(a, b), max(a, b)]
@@ -267,8 +275,9 @@ __device__ __forceinline__ StepCells start_cells(const QueryParams& P, float x, 
 // (x, then y, then z); more than kGridMaxVisit cells, or a NaN end point, fall
 // back to testing every box.  sc: cells of a on entry, of b on return.
 // PLANAR: z is ignored (a and b carry z = ws_min, grid cell 0).
-template <bool PLANAR = false>
-__device__ __forceinline__ bool step_free(const QueryParams& P, const GridView& grid, const float4* __restrict__ obs, uint32_t n_obs,
+// Grid: GridView or BlockGrid.
+template <bool PLANAR = false, typename Grid>
+__device__ __forceinline__ bool step_free(const QueryParams& P, const Grid& grid, const float4* __restrict__ obs, uint32_t n_obs,
                                           float ax, float ay, float az, float bx, float by, float bz, StepCells& sc, PropCount& cnt)
 {
     if(n_obs == 0) return true;
@@ -347,7 +356,8 @@ __device__ __forceinline__ int draw_steps(const QueryParams& P, float u)
 // reference's own formula (statePropagator.cu:97-99, (5v + 2ah) h / 6).
 // x0/x1 are sample rows [x y z vx vy vz ax ay az duration].
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ bool propagate_di(const QueryParams& P, const GridView& grid, const float* x0, const float* u, const float4* obs, uint32_t n_obs,
+template <typename Grid>
+__device__ __forceinline__ bool propagate_di(const QueryParams& P, const Grid& grid, const float* x0, const float* u, const float4* obs, uint32_t n_obs,
                                              float* x1, PropCount& cnt)
 {
     const float a0 = P.u_min[0] + u[0] * P.u_span[0];
@@ -436,7 +446,8 @@ __device__ __forceinline__ bool propagate_di(const QueryParams& P, const GridVie
 // so its sine and cosine are carried over.  Checks in the reference's order:
 // speed, pitch, workspace, obstacles.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ bool propagate_dubins(const QueryParams& P, const GridView& grid, const float* x0, const float* u, const float4* obs,
+template <typename Grid>
+__device__ __forceinline__ bool propagate_dubins(const QueryParams& P, const Grid& grid, const float* x0, const float* u, const float4* obs,
                                                  uint32_t n_obs, float* x1, PropCount& cnt)
 {
     const float a = P.u_min[0] + u[0] * P.u_span[0];
@@ -502,7 +513,8 @@ __device__ __forceinline__ bool propagate_dubins(const QueryParams& P, const Gri
 // as sin/cos of the portable pair.  Checks: workspace (x, y), then obstacles
 // in the plane (there is no speed check in the reference).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ bool propagate_unicycle(const QueryParams& P, const GridView& grid, const float* x0, const float* u, const float4* obs,
+template <typename Grid>
+__device__ __forceinline__ bool propagate_unicycle(const QueryParams& P, const Grid& grid, const float* x0, const float* u, const float4* obs,
                                                    uint32_t n_obs, float* x1, PropCount& cnt)
 {
     const float a = P.u_min[0] + u[0] * P.u_span[0];
@@ -581,7 +593,8 @@ __device__ __forceinline__ void quad_ode(const QueryParams& P, const float* s, f
     d[11] = fmaf(P.iiz, nc, fmaf(P.iiz * lmn, r, (P.jz * p) * q));
 }
 
-__device__ __forceinline__ bool propagate_quad(const QueryParams& P, const GridView& grid, const float* x0, const float* u, const float4* obs, uint32_t n_obs,
+template <typename Grid>
+__device__ __forceinline__ bool propagate_quad(const QueryParams& P, const Grid& grid, const float* x0, const float* u, const float4* obs, uint32_t n_obs,
                                                float* x1, PropCount& cnt)
 {
     const float zc = P.u_min[0] + u[0] * P.u_span[0];

@@ -439,8 +439,8 @@ __device__ __forceinline__ void with_model(int model, F&& f)
         if(MODELS == kBitUnicycle || model == KGMT_MODEL_UNICYCLE) f(std::integral_constant<int, KGMT_MODEL_UNICYCLE>{});
 }
 
-template <int MODEL>
-__device__ __forceinline__ bool propagate_model(const QueryParams& p, const GridView& grid, const float* x0, const float* u, const float4* obs,
+template <int MODEL, typename Grid>
+__device__ __forceinline__ bool propagate_model(const QueryParams& p, const Grid& grid, const float* x0, const float* u, const float4* obs,
                                                 uint32_t n_obs, float* x1, PropCount& cnt)
 {
     if constexpr(MODEL == KGMT_MODEL_QUADROTOR) return propagate_quad(p, grid, x0, u, obs, n_obs, x1, cnt);

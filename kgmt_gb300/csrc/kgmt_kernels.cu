@@ -27,6 +27,8 @@
 // iteration is built directly as two index lists -- re-activated old nodes
 // (repeat 1) followed by the nodes appended this iteration (repeat 15 or 1) --
 // which is the order the reference's scan over node indices produces.
+#include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <climits>
 #include <type_traits>
@@ -206,79 +208,113 @@ __global__ void k_admit(const QueryParams* __restrict__ P, QueryState* S, uint32
 }
 
 // ---------------------------------------------------------------------------
-// obstacle grid of one query per block: count boxes per cell, scan, fill.
-// A box is listed in every cell of [cell(min), cell(max)] per axis (ordered,
-// so an inverted box is still covered).  NaN coordinates, more boxes than
-// 16-bit indices hold, or more entries than the budget leave the grid marked
-// unusable and the propagate kernel tests every box.
+// Obstacle culling grid of n boxes, built by one block: count boxes per cell,
+// scan, fill.  A box is listed in every cell of [cell(min), cell(max)] per
+// axis (ordered, so an inverted box is still covered).  NaN coordinates, more
+// boxes than 16-bit indices hold, or more entries than `budget` leave the grid
+// unusable (false), and every box is tested.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_build_grid(const QueryParams* __restrict__ P, uint32_t first, uint32_t count,
-                                                    const uint32_t* __restrict__ slots)
+// The cells' 16-bit counters (two a word) become the fill cursors in place,
+// and a filled cell's cursor is the start of the next one: with a zero before
+// the first, they are the CSR starts.  Four lanes share a box, an x slice
+// each: a lane's chain of shared-memory atomics on a box's 8 to 30 cells is
+// the longest part of the build.
+constexpr uint32_t kGridBuildBytes = 16 + kGridCells * 2;  // shared memory of a build
+
+// calls f(o, cell) for the cells of the boxes o, this thread's share of them;
+// true when a box has a NaN coordinate (its cells are skipped)
+template <typename F>
+__device__ __forceinline__ bool for_box_cells(const QueryParams& p, const float4* obs, uint32_t n, F&& f)
 {
-    __shared__ uint32_t cnt[kGridCells];
-    __shared__ uint32_t scratch[34];
-    __shared__ int s_bad;
-    if(blockIdx.x >= count) return;
-    const QueryParams& p = P[slots ? slots[blockIdx.x] : first + blockIdx.x];
-    if(p.grid_start == nullptr) return;
-    const uint32_t n = p.n_obstacles;
-    for(uint32_t i = threadIdx.x; i < kGridCells; i += blockDim.x) cnt[i] = 0;
-    if(threadIdx.x == 0) s_bad = n > kMaxObstacles ? 1 : 0;
-    __syncthreads();
-    const int G = (int)p.grid_dim;
-    for(uint32_t o = threadIdx.x; o < n && !s_bad; o += blockDim.x)
+    constexpr int SHARE = 4, G = (int)kGridDim;
+    bool bad = false;
+#pragma unroll 1
+    for(uint32_t o = threadIdx.x / SHARE; o < n; o += blockDim.x / SHARE)
         {
-            const float4 a = p.obstacles[2 * o], b = p.obstacles[2 * o + 1];
+            const float4 a = obs[2 * o], b = obs[2 * o + 1];
             if(isnan(a.x) || isnan(a.y) || isnan(a.z) || isnan(b.x) || isnan(b.y) || isnan(b.z))
                 {
-                    s_bad = 1;
-                    break;
+                    bad = true;
+                    continue;
                 }
             const int x0 = grid_cell(p, fminf(a.x, b.x)), x1 = grid_cell(p, fmaxf(a.x, b.x));
             const int y0 = grid_cell(p, fminf(a.y, b.y)), y1 = grid_cell(p, fmaxf(a.y, b.y));
             const int z0 = p.planar ? 0 : grid_cell(p, fminf(a.z, b.z)), z1 = p.planar ? 0 : grid_cell(p, fmaxf(a.z, b.z));
-            for(int cx = x0; cx <= x1; ++cx)
+#pragma unroll 1
+            for(int cx = x0 + (int)(threadIdx.x % SHARE); cx <= x1; cx += SHARE)
+#pragma unroll 1
                 for(int cy = y0; cy <= y1; ++cy)
-                    for(int cz = z0; cz <= z1; ++cz) atomicAdd(&cnt[(cx * G + cy) * G + cz], 1u);
+                    for(int cz = z0; cz <= z1; ++cz) f(o, (cx * G + cy) * G + cz);
+        }
+    return bad;
+}
+
+// mem: kGridBuildBytes of shared memory, 16-byte aligned; scratch: 34 words;
+// items: shared or global memory.  All threads of the block (128 or 256) must
+// enter.  Returns the starts (kGridCells + 1 of them, inside mem; starts and
+// items are complete: the build ends with a block barrier), or nullptr when
+// the grid is unusable; *total gets the entries.
+__device__ __forceinline__ const uint16_t* build_grid(const QueryParams& p, const float4* obs, uint32_t n, uint32_t budget, char* mem,
+                                                      uint32_t* scratch, uint16_t* items, uint32_t* total)
+{
+    __shared__ int s_bad;
+    uint32_t* cursor = (uint32_t*)(mem + 16);  // cell c: half c & 1 of word c / 2
+    for(uint32_t i = threadIdx.x; i < kGridBuildBytes / 16; i += blockDim.x) ((uint4*)mem)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if(threadIdx.x < 34) scratch[threadIdx.x] = 0u;
+    if(threadIdx.x == 0) s_bad = n > kMaxObstacles ? 1 : 0;
+    __syncthreads();
+    const uint32_t boxes = n > kMaxObstacles ? 0u : n;
+    if(for_box_cells(p, obs, boxes, [&](uint32_t, int c) { atomicAdd(&cursor[c >> 1], 1u << ((c & 1) * 16)); })) s_bad = 1;
+    __syncthreads();
+    // counts -> exclusive prefixes; a thread owns 16 (or, of 128, 32)
+    // consecutive cells.  Pairs of 16-bit counts are summed in 32 bits.
+    const uint32_t words16 = kGridCells / 8 / blockDim.x;
+    uint4* own = (uint4*)cursor + threadIdx.x * words16;
+    uint32_t local = 0;
+    for(uint32_t i = 0; i < words16; ++i)
+        {
+            const uint4 v = own[i];
+            local += (v.x & 0xffffu) + (v.x >> 16) + (v.y & 0xffffu) + (v.y >> 16) + (v.z & 0xffffu) + (v.z >> 16) + (v.w & 0xffffu) + (v.w >> 16);
+        }
+    uint32_t run = block_exclusive_scan<256>(local, scratch, total);
+    if(s_bad || *total > budget || *total > kMaxGridItems) return nullptr;
+    for(uint32_t i = 0; i < words16; ++i)
+        {
+            uint4 v = own[i];
+            auto prefix = [&](uint32_t w) {
+                const uint32_t lo = run, hi = run + (w & 0xffffu);
+                run = hi + (w >> 16);
+                return lo | (hi << 16);
+            };
+            v.x = prefix(v.x), v.y = prefix(v.y), v.z = prefix(v.z), v.w = prefix(v.w);
+            own[i] = v;
         }
     __syncthreads();
-    // exclusive scan: thread t owns cells [16 t, 16 t + 16)
-    constexpr int PER = kGridCells / 256;
-    uint32_t local = 0;
-    if(threadIdx.x < 256)
-        for(int i = 0; i < PER; ++i) local += cnt[threadIdx.x * PER + i];
-    uint32_t total;
-    uint32_t run = block_exclusive_scan<256>(local, scratch, &total);
-    for(int i = 0; i < PER; ++i)
-        {
-            const uint32_t c = threadIdx.x * PER + i;
-            const uint32_t k = cnt[c];
-            p.grid_start[c] = (uint16_t)run;  // meaningful only when usable (total <= 65535)
-            cnt[c] = run;  // becomes the fill cursor
-            run += k;
-        }
-    const bool usable = !s_bad && total <= p.grid_budget && total <= kMaxGridItems;
+    for_box_cells(p, obs, boxes, [&](uint32_t o, int c) {
+        const int sh = (c & 1) * 16;
+        items[(atomicAdd(&cursor[c >> 1], 1u << sh) >> sh) & 0xffffu] = (uint16_t)o;
+    });
+    __syncthreads();
+    return (const uint16_t*)cursor - 1;
+}
+
+// the culling grid of one query per block
+__global__ void __launch_bounds__(256) k_build_grid(const QueryParams* __restrict__ P, uint32_t first, uint32_t count,
+                                                    const uint32_t* __restrict__ slots)
+{
+    __shared__ alignas(16) char mem[kGridBuildBytes];
+    __shared__ uint32_t scratch[34];
+    if(blockIdx.x >= count) return;
+    const QueryParams& p = P[slots ? slots[blockIdx.x] : first + blockIdx.x];
+    if(p.grid_start == nullptr) return;
+    uint32_t total = 0;
+    const uint16_t* start = build_grid(p, p.obstacles, p.n_obstacles, p.grid_budget, mem, scratch, p.grid_items, &total);
+    if(start)
+        for(uint32_t c = threadIdx.x; c <= kGridCells; c += 256) p.grid_start[c] = start[c];
     if(threadIdx.x == 0)
         {
-            p.grid_start[kGridCells] = (uint16_t)total;
             p.grid_meta[0] = total;
-            p.grid_meta[1] = usable ? 1u : 0u;
-        }
-    __syncthreads();
-    if(!usable) return;
-    for(uint32_t o = threadIdx.x; o < n; o += blockDim.x)
-        {
-            const float4 a = p.obstacles[2 * o], b = p.obstacles[2 * o + 1];
-            const int x0 = grid_cell(p, fminf(a.x, b.x)), x1 = grid_cell(p, fmaxf(a.x, b.x));
-            const int y0 = grid_cell(p, fminf(a.y, b.y)), y1 = grid_cell(p, fmaxf(a.y, b.y));
-            const int z0 = p.planar ? 0 : grid_cell(p, fminf(a.z, b.z)), z1 = p.planar ? 0 : grid_cell(p, fmaxf(a.z, b.z));
-            for(int cx = x0; cx <= x1; ++cx)
-                for(int cy = y0; cy <= y1; ++cy)
-                    for(int cz = z0; cz <= z1; ++cz)
-                        {
-                            const uint32_t pos = atomicAdd(&cnt[(cx * G + cy) * G + cz], 1u);
-                            p.grid_items[pos] = (uint16_t)o;
-                        }
+            p.grid_meta[1] = start ? 1u : 0u;
         }
 }
 
@@ -701,31 +737,167 @@ __global__ void k_stage_obstacles(const float* __restrict__ src, float4* dst, ui
 }
 
 // ---------------------------------------------------------------------------
-// function-level propagation with explicit uniforms
+// function-level propagation with explicit uniforms: sample rows [n][D] and
+// eight uniforms a sample in, end rows, verdicts and region ids out
 // ---------------------------------------------------------------------------
-__global__ void k_propagate_samples(const QueryParams p, const float* __restrict__ x0, const float* __restrict__ uni,
-                                    const float* __restrict__ obs_rows, uint32_t n_obs, uint32_t n, float* x1, uint8_t* valid,
-                                    int32_t* r1, int32_t* r2)
+// Each block stages the boxes, builds the culling grid over them in its own
+// shared memory where that pays (no workspace, nothing shared between calls)
+// and runs a contiguous share of the samples.  Two forms:
+//   one sample a thread, blocks of 128 (four warps load the four schedulers of
+//   an SM evenly): up to 256 samples per resident block, where a call's time is
+//   its slowest sample's;
+//   sorted, blocks of 256: each share is counting-sorted by step count, 1024
+//   samples at a time, and the runs of 32 are taken longest first by whichever
+//   warp is free, so a warp's lanes loop equally long.
+// End rows leave through a per-warp stage, so that a warp's stores cover whole
+// rows.  Bound by instruction issue (the model's step).  Against one kernel for
+// all models that ran one unsorted sample a thread and tested every box at
+// every step: 2^20 quadrotor samples in 200 boxes 352 us, 1631 before; 200,000
+// Dubins samples in 50 boxes 26 us, 60 before; 1000 double-integrator samples
+// in 10 boxes (latency) 4.4 us, 5.0 before.
+constexpr uint32_t kSamplesChunk = 1024;  // samples sorted at a time
+// dynamic shared memory of the largest call (boxes; the grid's starts and
+// items); the static arrays stay below the 22 KB left of an SM's 227
+constexpr size_t kSamplesSmemMax = 205 * 1024;
+// grid entries a block holds (scenes with more test every box): 8 a box, which
+// boxes of the workloads' sizes stay below, within the shared memory there is
+static uint32_t samples_items(uint32_t n_obs)
 {
-    extern __shared__ float4 s_obs[];
-    const int w = p.planar ? 2 : 3;
-    for(uint32_t i = threadIdx.x; i < n_obs; i += blockDim.x) stage_box(obs_rows + (size_t)i * 2 * w, w, s_obs + 2 * i);
+    const size_t room = (kSamplesSmemMax - (size_t)n_obs * 32 - kGridBuildBytes) / 2;
+    return (uint32_t)std::min<size_t>(std::max<size_t>(4096, (size_t)n_obs * 8), std::min<size_t>(room, kMaxGridItems));
+}
+static size_t samples_smem(uint32_t n_obs, uint32_t items) { return (size_t)n_obs * 32 + (items ? kGridBuildBytes + (size_t)items * 2 : 0); }
+constexpr int samples_threads(bool sorted) { return sorted ? 256 : 128; }
+// blocks per SM that the kernel is compiled for.  One sample a thread: no
+// spills before warps (1000 double-integrator samples 4.4 us at 3 blocks, 5.0
+// at 4).  Sorted: the quadrotor keeps its state in 128 registers, the other
+// models trade a few spills for more warps (2^20 double-integrator samples in
+// 20 boxes 66 us at 3 blocks, 76 at 2).
+constexpr int samples_blocks(int model, bool sorted) { return !sorted ? 3 : model == KGMT_MODEL_QUADROTOR ? 2 : 3; }
+
+template <int MODEL, bool SORTED>
+__global__ void __launch_bounds__(samples_threads(SORTED), samples_blocks(MODEL, SORTED))
+  k_propagate_samples(const __grid_constant__ QueryParams p, const float* x0, const float* __restrict__ uni, const float* __restrict__ obs_rows,
+                      uint32_t n_obs, uint32_t n, uint32_t share, uint32_t grid_items, float* x1, uint8_t* valid, int32_t* r1, int32_t* r2)
+{
+    constexpr int D = ModelDims<MODEL>::D, NC = ModelDims<MODEL>::NC;
+    constexpr uint32_t NT = (uint32_t)samples_threads(SORTED);
+    extern __shared__ float4 s_dyn[];
+    float4* s_obs = s_dyn;
+    char* s_grid = (char*)(s_dyn + 2 * (size_t)n_obs);
+    uint16_t* s_items = (uint16_t*)(s_grid + kGridBuildBytes);
+    __shared__ float s_stage[NT * D];
+    __shared__ uint32_t s_scan[34];
+    __shared__ uint32_t s_hist[kSortBins];
+    __shared__ uint16_t s_perm[SORTED ? kSamplesChunk : 1];
+    __shared__ uint32_t s_next;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t b0 = min(n, blockIdx.x * share), b1 = min(n, b0 + share);
+    float a[D], u[8];
+    auto load = [&](uint32_t s) {
+#pragma unroll
+        for(int j = 0; j < D; ++j) a[j] = x0[(size_t)s * D + j];
+#pragma unroll
+        for(int j = 0; j < NC + 1; ++j) u[j] = uni[(size_t)s * 8 + j];
+    };
+    // one run a warp: its rows are on their way while the boxes are staged
+    if(!SORTED && b0 + threadIdx.x < b1) load(b0 + threadIdx.x);
+    const int w = MODEL == KGMT_MODEL_UNICYCLE ? 2 : 3;
+    for(uint32_t i = threadIdx.x; i < n_obs; i += NT) stage_box(obs_rows + (size_t)i * 2 * w, w, s_obs + 2 * i);
     __syncthreads();
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if(s >= n) return;
-    const int D = (int)p.sample_dim;
-    float a[kMaxSampleDim], b[kMaxSampleDim], u[8];
-    for(int j = 0; j < D; ++j) a[j] = x0[(size_t)s * D + j];
-    for(int j = 0; j < 8; ++j) u[j] = uni[(size_t)s * 8 + j];
-    PropCount cnt;
-    const GridView none{nullptr, nullptr, nullptr};
-    bool ok = false;
-    with_model<kAllModels>(p.model, [&](auto m) { ok = propagate_model<decltype(m)::value>(p, none, a, u, s_obs, n_obs, b, cnt); });
-    for(int j = 0; j < D; ++j) x1[(size_t)s * D + j] = b[j];
-    valid[s] = ok ? 1 : 0;
-    const CellIds c = cell_ids(p, b);
-    if(r1) r1[s] = c.r1;
-    if(r2) r2[s] = c.r2;
+    BlockGrid grid{nullptr, s_items};
+    if(grid_items)
+        {
+            uint32_t total;
+            grid.start = build_grid(p, s_obs, n_obs, grid_items, s_grid, s_scan, s_items, &total);
+        }
+    const unsigned full = 0xffffffffu;
+    float* stage = s_stage + warp * 32 * D;
+    for(uint32_t c0 = b0; c0 < b1; c0 += kSamplesChunk)
+        {
+            const uint32_t cn = min(kSamplesChunk, b1 - c0);
+            const uint32_t n_runs = (cn + 31u) / 32u;
+            if(SORTED)
+                {
+                    constexpr int PER = (int)kSamplesChunk / NT;
+                    uint32_t key[PER], rank[PER];
+                    if(threadIdx.x < kSortBins) s_hist[threadIdx.x] = 0;
+                    if(threadIdx.x == 0) s_next = 0;
+                    __syncthreads();
+#pragma unroll
+                    for(int h = 0; h < PER; ++h)
+                        {
+                            const uint32_t i = (uint32_t)h * NT + threadIdx.x;
+                            key[h] = kSortBins - 1;
+                            if(i < cn)
+                                {
+                                    const int k = draw_steps(p, uni[(size_t)(c0 + i) * 8 + NC]);
+                                    key[h] = k < kSortBins - 1 ? (k > 0 ? (uint32_t)k : 0u) : kSortBins - 2;
+                                    rank[h] = atomicAdd(&s_hist[key[h]], 1u);
+                                }
+                        }
+                    __syncthreads();
+                    if(threadIdx.x < 32)
+                        {
+                            const uint32_t v = s_hist[threadIdx.x];
+                            uint32_t x = v;
+#pragma unroll
+                            for(int o = 1; o < 32; o <<= 1)
+                                {
+                                    const uint32_t y = __shfl_up_sync(full, x, o);
+                                    if(lane >= (uint32_t)o) x += y;
+                                }
+                            s_hist[threadIdx.x] = x - v;
+                        }
+                    __syncthreads();
+#pragma unroll
+                    for(int h = 0; h < PER; ++h)
+                        {
+                            const uint32_t i = (uint32_t)h * NT + threadIdx.x;
+                            if(i < cn) s_perm[s_hist[key[h]] + rank[h]] = (uint16_t)i;
+                        }
+                    __syncthreads();
+                }
+            for(uint32_t run = warp;;)
+                {
+                    if(SORTED)
+                        {
+                            if(lane == 0) run = atomicAdd(&s_next, 1u);
+                            run = __shfl_sync(full, run, 0);
+                        }
+                    if(run >= n_runs) break;
+                    // longest runs first
+                    const uint32_t slot = (SORTED ? n_runs - 1u - run : run) * 32u + lane;
+                    const bool live = slot < cn;
+                    const uint32_t s = c0 + (live ? (SORTED ? (uint32_t)s_perm[slot] : slot) : 0u);
+                    if(live)
+                        {
+                            float b[D];
+                            if(SORTED) load(s);
+                            PropCount cnt;
+                            const bool ok = propagate_model<MODEL>(p, grid, a, u, s_obs, n_obs, b, cnt);
+                            valid[s] = ok ? 1 : 0;
+                            const CellIds c = cell_ids(p, b);
+                            if(r1) r1[s] = c.r1;
+                            if(r2) r2[s] = c.r2;
+#pragma unroll
+                            for(int j = 0; j < D; ++j) stage[lane * D + j] = b[j];
+                        }
+                    __syncwarp();
+                    const uint32_t rows = min(32u, cn - (slot - lane));
+                    // element e of the stage is column e % D of row e / D
+#pragma unroll
+                    for(uint32_t i = 0; i < (uint32_t)D; ++i)
+                        {
+                            const uint32_t e = i * 32u + lane, row = e / D;
+                            const uint32_t rs = __shfl_sync(full, s, row & 31u);
+                            if(row < rows) x1[(size_t)rs * D + (e - row * D)] = stage[e];
+                        }
+                    __syncwarp();
+                    if(!SORTED) break;  // one run a warp
+                }
+            __syncthreads();
+        }
 }
 
 // ---------------------------------------------------------------------------
@@ -935,18 +1107,77 @@ cudaError_t launch_tail(const LaunchArgs& a, TailScratch* ts, int models, int gr
         }
 }
 
+template <int MODEL, bool SORTED>
+static cudaError_t launch_samples_t(const QueryParams& p, const float* x0, const float* u, const float* obs, uint32_t n_obs, uint32_t n,
+                                    uint32_t share, uint32_t items, float* x1, uint8_t* valid, int32_t* r1, int32_t* r2, cudaStream_t s)
+{
+    const size_t smem = samples_smem(n_obs, items);
+    if(smem > 26 * 1024)
+        {
+            // more than 48 KB with the static arrays (always the same limit,
+            // so that calls from several threads agree)
+            const cudaError_t e = cudaFuncSetAttribute(k_propagate_samples<MODEL, SORTED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       (int)kSamplesSmemMax);
+            if(e != cudaSuccess) return e;
+        }
+    k_propagate_samples<MODEL, SORTED><<<(n + share - 1) / share, samples_threads(SORTED), smem, s>>>(p, x0, u, obs, n_obs, n, share, items, x1,
+                                                                                                     valid, r1, r2);
+    return cudaGetLastError();
+}
+
+// SMs of the current device, asked for once per device (a property that does
+// not change; two threads asking at once store the same number)
+static cudaError_t current_sms(int* sms)
+{
+    static std::atomic<int> known[64];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if(e != cudaSuccess) return e;
+    const bool kept = dev >= 0 && dev < 64;
+    if(kept && (*sms = known[dev].load(std::memory_order_relaxed)) > 0) return cudaSuccess;
+    e = cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev);
+    if(e == cudaSuccess && kept) known[dev].store(*sms, std::memory_order_relaxed);
+    return e;
+}
+
+template <int MODEL>
+static cudaError_t launch_samples_m(const QueryParams& p, const float* x0, const float* u, const float* obs, uint32_t n_obs, uint32_t n, float* x1,
+                                    uint8_t* valid, int32_t* r1, int32_t* r2, cudaStream_t s)
+{
+    int sms = 0;
+    const cudaError_t e = current_sms(&sms);
+    if(e != cudaSuccess) return e;
+    // The grid is built when the box tests it saves cost more than it does: a
+    // test is about 12 instructions a step, the cell walk about as much as 10
+    // tests, and the build about 5500 cycles, while the samples take
+    // n / (128 SMs) rounds of one warp per scheduler.  Measured without / with
+    // the grid (before the two forms were split): 8193 Dubins samples in 100
+    // boxes 17.8 / 15.4 us, 30 boxes 9.9 / 12.3; 49,999 in 50 boxes 20.9 /
+    // 17.4, 20 boxes 12.8 / 15.7; 2^20 in 20 boxes 124 / 105.
+    const double rounds = std::max(1.0, n / (128.0 * sms)), steps = 0.5 * (p.min_steps + p.max_steps);
+    const uint32_t items = rounds * steps * 12.0 * ((double)n_obs - 10.0) > 5500.0 ? samples_items(n_obs) : 0u;
+    // sorted shares once the samples fill the resident blocks more than once
+    // (200,000 quadrotor samples in 50 boxes: 73 us sorted, 148 unsorted)
+    const uint32_t per_sm =
+      (uint32_t)std::max<size_t>(1, std::min<size_t>((size_t)samples_blocks(MODEL, true), 227 * 1024 / (samples_smem(n_obs, items) + 22 * 1024)));
+    const uint32_t blocks = (uint32_t)sms * per_sm;
+    if(n <= blocks * (uint32_t)samples_threads(true))
+        return launch_samples_t<MODEL, false>(p, x0, u, obs, n_obs, n, (uint32_t)samples_threads(false), items, x1, valid, r1, r2, s);
+    const uint32_t share = ((n + blocks - 1) / blocks + 31u) & ~31u;
+    return launch_samples_t<MODEL, true>(p, x0, u, obs, n_obs, n, share, items, x1, valid, r1, r2, s);
+}
+
 cudaError_t launch_propagate_samples(const QueryParams& p, const float* x0, const float* u, const float* obs, uint32_t n_obs, uint32_t n,
                                      float* x1, uint8_t* valid, int32_t* r1, int32_t* r2, cudaStream_t s)
 {
     if(n == 0) return cudaSuccess;
-    const size_t smem = (size_t)n_obs * 2 * sizeof(float4);
-    if(smem > 48 * 1024)
+    switch(p.model)
         {
-            cudaError_t e = cudaFuncSetAttribute(k_propagate_samples, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if(e != cudaSuccess) return e;
+            case KGMT_MODEL_QUADROTOR: return launch_samples_m<KGMT_MODEL_QUADROTOR>(p, x0, u, obs, n_obs, n, x1, valid, r1, r2, s);
+            case KGMT_MODEL_DUBINS_AIRPLANE: return launch_samples_m<KGMT_MODEL_DUBINS_AIRPLANE>(p, x0, u, obs, n_obs, n, x1, valid, r1, r2, s);
+            case KGMT_MODEL_UNICYCLE: return launch_samples_m<KGMT_MODEL_UNICYCLE>(p, x0, u, obs, n_obs, n, x1, valid, r1, r2, s);
+            default: return launch_samples_m<KGMT_MODEL_DOUBLE_INTEGRATOR>(p, x0, u, obs, n_obs, n, x1, valid, r1, r2, s);
         }
-    k_propagate_samples<<<(n + 127) / 128, 128, smem, s>>>(p, x0, u, obs, n_obs, n, x1, valid, r1, r2);
-    return cudaGetLastError();
 }
 
 }  // namespace kgmt
