@@ -6,7 +6,9 @@ calls fail with an exception carrying ``kgmt_last_error()``.
 from __future__ import annotations
 
 import ctypes as C
+import operator
 import os
+import struct
 from pathlib import Path
 
 from .config import PlannerConfig
@@ -92,7 +94,23 @@ class KgmtServerOptions(C.Structure):
                 ("propagate_block", C.c_uint32)]
 
 
+# the struct's fields in one pack: 1.5 us a config instead of 5.8 by one ctypes
+# assignment a field, which was half of a small propagate_samples call
+_PACK = struct.Struct("@iiIIIIIfffffIIff4f4ffffffffQfffI")
+assert _PACK.size == C.sizeof(KgmtConfig)
+_NAMES = [n for n, _ in KgmtConfig._fields_]
+_BEFORE_U = operator.attrgetter(*_NAMES[:_NAMES.index("u_min")])
+_AFTER_U = operator.attrgetter(*_NAMES[_NAMES.index("u_max") + 1:])
+
+
 def to_c(cfg: PlannerConfig) -> KgmtConfig:
+    # whole numbers in range and four-element bounds; anything else takes the
+    # field-by-field way with ctypes' own conversions and refusals
+    try:
+        if len(cfg.u_min) == len(cfg.u_max) == 4:
+            return KgmtConfig.from_buffer_copy(_PACK.pack(*_BEFORE_U(cfg), *cfg.u_min, *cfg.u_max, *_AFTER_U(cfg)))
+    except (struct.error, OverflowError, TypeError, ValueError):
+        pass
     k = KgmtConfig()
     for name, _ in KgmtConfig._fields_:
         v = getattr(cfg, name)
