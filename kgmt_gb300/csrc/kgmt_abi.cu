@@ -201,12 +201,14 @@ static kgmt_status plan_setup(kgmt_planner* p, const float* h_initial, const flo
     size_t off = 0;
     RETURN_IF(!p->arena.alloc(L.total, &off), KGMT_ERR_OOM, std::string(who) + ": arena allocation failed");
     p->params = make_params(p->cfg, h_initial, h_goal, p->arena.base() + off, L, nullptr, n_obstacles);
-    CHECK_ST(cuda_status(launch_stage_obstacles(d_obstacles, p->params.obstacles, n_obstacles, (int)ws_dims_of(p->cfg.model), p->eng.stream()),
-                         "stage obstacles"));
-    p->eng.host_params(0) = p->params;
+    // the boxes are staged by the admission launch
+    p->params.raw_obstacles = n_obstacles ? d_obstacles : nullptr;
+    p->params.raw_w = (int32_t)ws_dims_of(p->cfg.model);
     p->eng.set_models(Engine::model_bit(p->cfg.model));
     p->eng.set_max_obstacles(n_obstacles);
-    return p->eng.admit(0, 1, 1);
+    const kgmt_status st = p->eng.admit_only(p->params);
+    p->params.raw_obstacles = nullptr;  // the caller's array
+    return st;
 }
 
 extern "C" kgmt_status kgmt_plan(kgmt_planner* p, const float* h_initial, const float* h_goal, const float* d_obstacles,
@@ -214,9 +216,8 @@ extern "C" kgmt_status kgmt_plan(kgmt_planner* p, const float* h_initial, const 
 {
     CHECK_ST(plan_setup(p, h_initial, h_goal, d_obstacles, n_obstacles, "kgmt_plan"));
     CHECK_ST(p->eng.run_until_done(p->cfg.max_iterations));
-    CHECK_ST(p->eng.extract_paths(1));
     uint32_t err = 0;
-    CHECK_ST(p->eng.read_states_and_error(0, 1, &p->state, &err));
+    CHECK_ST(p->eng.finish(1, &p->state, &err));
     RETURN_IF(err != 0, KGMT_ERR_TIMEOUT, "kgmt_plan: a device-side wait gave up (error bits " + std::to_string(err) + ")");
     RETURN_IF(bounds_error_take() != 0, KGMT_ERR_INTERNAL, "kgmt_plan: an index check failed (bounds-checked build)");
     p->planned = true;
@@ -338,17 +339,22 @@ static kgmt_status copy_tree_common(const QueryParams& prm, const QueryState& st
     return cuda_status(cudaStreamSynchronize(s), "sync");
 }
 
-static kgmt_status copy_path_common(const QueryParams& prm, const QueryState& st, cudaStream_t s, float* h_rows, uint32_t max_rows,
+// the path's rows: from the host path buffer where they are there, else from
+// the query's own buffer
+static kgmt_status copy_path_common(const Engine& eng, const QueryParams& prm, const QueryState& st, float* h_rows, uint32_t max_rows,
                                     uint32_t* n_rows)
 {
     const uint32_t n = st.path_len < max_rows ? st.path_len : max_rows;
     if(n_rows) *n_rows = n;
-    if(n && h_rows)
+    if(!n || !h_rows) return KGMT_OK;
+    const size_t bytes = (size_t)n * prm.sample_dim * 4;
+    if(const float* rows = eng.host_path(st))
         {
-            CHECK_ST(cuda_status(cudaMemcpyAsync(h_rows, prm.path, (size_t)n * prm.sample_dim * 4, cudaMemcpyDeviceToHost, s), "copy path"));
-            return cuda_status(cudaStreamSynchronize(s), "sync");
+            std::memcpy(h_rows, rows, bytes);
+            return KGMT_OK;
         }
-    return KGMT_OK;
+    CHECK_ST(cuda_status(cudaMemcpyAsync(h_rows, prm.path, bytes, cudaMemcpyDeviceToHost, eng.stream()), "copy path"));
+    return cuda_status(cudaStreamSynchronize(eng.stream()), "sync");
 }
 
 extern "C" kgmt_status kgmt_copy_tree(kgmt_planner* p, float* h_samples, int32_t* h_parents, float* h_costs, uint32_t max_nodes)
@@ -362,7 +368,7 @@ extern "C" kgmt_status kgmt_copy_path(kgmt_planner* p, float* h_rows, uint32_t m
 {
     RETURN_IF(!p, KGMT_ERR_INVALID_ARG, "kgmt_copy_path: NULL planner");
     RETURN_IF(!p->planned, KGMT_ERR_NOT_READY, "kgmt_copy_path: no plan has completed");
-    return copy_path_common(p->params, p->state, p->eng.stream(), h_rows, max_rows, n_rows);
+    return copy_path_common(p->eng, p->params, p->state, h_rows, max_rows, n_rows);
 }
 
 extern "C" kgmt_status kgmt_device_tree(kgmt_planner* p, const float** d_samples, const int32_t** d_parents, const float** d_costs)
@@ -470,10 +476,9 @@ static kgmt_status batch_run(kgmt_batch* b, uint32_t n, const kgmt_config* cfgs,
     const uint32_t it0 = b->eng.iterations_launched();
     CHECK_ST(b->eng.admit(0, n, n, d_inits, d_goals));
     CHECK_ST(b->eng.run_until_done(max_iters));
-    CHECK_ST(b->eng.extract_paths(n));
     b->states.resize(n);
     uint32_t err = 0;
-    CHECK_ST(b->eng.read_states_and_error(0, n, b->states.data(), &err));
+    CHECK_ST(b->eng.finish(n, b->states.data(), &err));
     b->n_last = n;
     RETURN_IF(err != 0, KGMT_ERR_TIMEOUT, "batch: a device-side wait gave up (error bits " + std::to_string(err) + ")");
     RETURN_IF(bounds_error_take() != 0, KGMT_ERR_INTERNAL, "batch: an index check failed (bounds-checked build)");
@@ -568,7 +573,7 @@ extern "C" kgmt_status kgmt_batch_copy_path(kgmt_batch* b, uint32_t i, float* h_
 {
     RETURN_IF(!b, KGMT_ERR_INVALID_ARG, "kgmt_batch_copy_path: NULL batch");
     RETURN_IF(i >= b->n_last, KGMT_ERR_NOT_READY, "kgmt_batch_copy_path: no such query in the last batch");
-    return copy_path_common(b->params[i], b->states[i], b->eng.stream(), h_rows, max_rows, n_rows);
+    return copy_path_common(b->eng, b->params[i], b->states[i], h_rows, max_rows, n_rows);
 }
 
 extern "C" kgmt_status kgmt_batch_autotune(kgmt_batch* b, uint32_t n, const kgmt_config* cfgs, const float* h_inits, const float* h_goals,
@@ -750,7 +755,7 @@ extern "C" kgmt_status kgmt_server_create(const kgmt_server_options* opt, void* 
     s->opt = *opt;
     if(s->opt.iters_per_step == 0) s->opt.iters_per_step = 1;
     // one graph replay per step: a unit of iters_per_step iterations
-    kgmt_status st = s->eng.init(opt->max_slots, (cudaStream_t)stream, opt->propagate_block ? opt->propagate_block : 256, s->opt.iters_per_step, true);
+    kgmt_status st = s->eng.init(opt->max_slots, (cudaStream_t)stream, opt->propagate_block ? opt->propagate_block : 256, s->opt.iters_per_step, true, false);
     if(st == KGMT_OK) st = s->arena.reserve(opt->memory_budget);
     if(st == KGMT_OK) st = s->eng.set_active(opt->max_slots);
     if(st == KGMT_OK) st = cuda_status(cudaEventCreateWithFlags(&s->ev, cudaEventDisableTiming), "cudaEventCreate");

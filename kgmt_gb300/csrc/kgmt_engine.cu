@@ -362,7 +362,11 @@ kgmt_result to_result(const QueryState& s, uint64_t ticket)
 // ---------------------------------------------------------------------------
 // engine
 // ---------------------------------------------------------------------------
-__global__ void k_set_n_slots(Sched* sched, uint32_t n) { sched->n_slots = n; }
+__global__ void k_set_n_slots(Sched* sched, uint32_t n)
+{
+    sched->n_slots = n;
+    sched->path_words = 0;
+}
 
 __global__ void k_set_endpoints(QueryParams* P, uint32_t first, uint32_t count, const float* __restrict__ inits,
                                 const float* __restrict__ goals)
@@ -394,7 +398,7 @@ Engine::~Engine()
 
 LaunchArgs Engine::args() const { return LaunchArgs{d_params_, d_states_, d_sched_, d_tile_a_, d_tile_c_, d_tile_old_}; }
 
-kgmt_status Engine::init(uint32_t slots, cudaStream_t stream, uint32_t prop_block, uint32_t iters_per_graph, bool use_graph)
+kgmt_status Engine::init(uint32_t slots, cudaStream_t stream, uint32_t prop_block, uint32_t iters_per_graph, bool use_graph, bool host_paths)
 {
     int dev_count = 0;
     if(cudaGetDeviceCount(&dev_count) != cudaSuccess || dev_count == 0)
@@ -443,7 +447,18 @@ kgmt_status Engine::init(uint32_t slots, cudaStream_t stream, uint32_t prop_bloc
     KGMT_CUDA(cudaHostAlloc((void**)&h_running_, sizeof(uint32_t) * 4, cudaHostAllocMapped), "cudaHostAlloc(mapped)");
     std::memset(h_running_, 0, sizeof(uint32_t) * 4);
     KGMT_CUDA(cudaHostGetDevicePointer((void**)&d_running_, h_running_, 0), "cudaHostGetDevicePointer");
-    KGMT_CUDA(cudaMallocHost((void**)&h_stage_states_, sizeof(QueryState) * slots), "cudaMallocHost(states)");
+    // the states and, packed, the rows of the paths found, as k_paths leaves
+    // them: one pinned block (2 KiB of path a slot: 50 rows of the double
+    // integrator, 30 of the quadrotor; what does not fit is copied on demand)
+    {
+        const size_t state_bytes = (sizeof(QueryState) * slots + 255) & ~size_t(255);
+        const size_t path_bytes = host_paths ? std::min<size_t>(std::max<size_t>((size_t)slots * 2048, 32768), size_t(16) << 20) : 0;
+        KGMT_CUDA(cudaHostAlloc((void**)&h_stage_states_, state_bytes + path_bytes, cudaHostAllocMapped), "cudaHostAlloc(states)");
+        char* dev = nullptr;
+        KGMT_CUDA(cudaHostGetDevicePointer((void**)&dev, h_stage_states_, 0), "cudaHostGetDevicePointer");
+        h_paths_ = (const float*)((const char*)h_stage_states_ + state_bytes);
+        sink_ = HostSink{(QueryState*)dev, d_running_ + 1, host_paths ? (float*)(dev + state_bytes) : nullptr, (uint32_t)(path_bytes / 4)};
+    }
     for(auto& e : ev_) KGMT_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
     return set_prop_block(prop_block ? prop_block : 256);
 }
@@ -578,6 +593,23 @@ kgmt_status Engine::admit(uint32_t first, uint32_t count, uint32_t n_active, con
     return st;
 }
 
+kgmt_status Engine::admit_only(const QueryParams& p)
+{
+    NvtxRange r("kgmt admit");
+    if(slots_ != 1)
+        {
+            set_error("admit_only: the engine holds more than one query");
+            return KGMT_ERR_INTERNAL;
+        }
+    h_params_[0] = p;
+    h_params_[0].raw_obstacles = nullptr;
+    n_active_ = 1;
+    KGMT_CUDA(launch_begin(args(), p, d_tail_, stream_), "k_begin");
+    launches_ += 1;
+    bar_zero_ = true;
+    return KGMT_OK;
+}
+
 kgmt_status Engine::record_event(cudaEvent_t* out)
 {
     if(prof_used_ >= prof_events_.size())
@@ -646,17 +678,25 @@ kgmt_status Engine::run_tail(bool* done, bool* declined_at_once)
             if(st != KGMT_OK) return st;
             prof_kind_.push_back(1);
         }
-    KGMT_CUDA(launch_tail(args(), d_tail_, models_, tail_grid_[models_], smem_boxes_, tail_max_samples_, d_running_ + 2, stream_), "k_tail");
+    KGMT_CUDA(launch_tail(args(), d_tail_, models_, tail_grid_[models_], smem_boxes_, tail_max_samples_, d_running_ + 2, !bar_zero_, stream_),
+              "k_tail");
+    bar_zero_ = false;
     if(profile_)
         {
             kgmt_status st = record_event(nullptr);
             if(st != KGMT_OK) return st;
         }
     launches_ += 1;
+    // most tail launches finish their queries: the paths and the states for
+    // the host are queued behind without waiting to know (queries still
+    // running are left alone)
+    kgmt_status ps = extract_paths(n_active_);
+    if(ps != KGMT_OK) return ps;
     KGMT_CUDA(cudaStreamSynchronize(stream_), "cudaStreamSynchronize");
     volatile uint32_t* w = h_running_;
     tail_iters_ += w[2];
     *done = w[0] == 0u;
+    results_ready_ = *done;
     *declined_at_once = w[3] != 0u && w[2] == 0u;
     return KGMT_OK;
 }
@@ -731,6 +771,7 @@ kgmt_status Engine::run_until_done(uint32_t max_iters)
     // that could not take even one iteration, the next attempt waits twice as
     // many units).
     NvtxRange r("kgmt run until done");
+    results_ready_ = false;
     const uint32_t G = iters_per_graph_;
     const uint32_t max_units = (max_iters + G - 1) / G + 2;
     volatile uint32_t* running = h_running_;
@@ -866,8 +907,26 @@ kgmt_status Engine::read_states_and_error(uint32_t first, uint32_t count, QueryS
 kgmt_status Engine::extract_paths(uint32_t n_active)
 {
     NvtxRange r("kgmt paths");
-    KGMT_CUDA(launch_paths(args(), n_active, stream_), "k_paths");
+    KGMT_CUDA(launch_paths(args(), n_active, sink_, stream_), "k_paths");
     launches_ += 1;
+    return KGMT_OK;
+}
+
+kgmt_status Engine::finish(uint32_t count, QueryState* out, uint32_t* err)
+{
+    if(count > n_active_)
+        {
+            set_error("finish: slot range out of bounds");
+            return KGMT_ERR_INVALID_ARG;
+        }
+    if(!results_ready_)
+        {
+            kgmt_status st = extract_paths(count);
+            if(st != KGMT_OK) return st;
+            KGMT_CUDA(cudaStreamSynchronize(stream_), "cudaStreamSynchronize");
+        }
+    if(count) std::memcpy(out, h_stage_states_, sizeof(QueryState) * count);
+    *err = h_running_[1];
     return KGMT_OK;
 }
 

@@ -67,7 +67,8 @@ kgmt_result to_result(const QueryState& s, uint64_t ticket);
 class Engine {
    public:
     ~Engine();
-    kgmt_status init(uint32_t slots, cudaStream_t stream, uint32_t prop_block, uint32_t iters_per_graph, bool use_graph);
+    // host_paths: keep a pinned buffer that the found paths are left in
+    kgmt_status init(uint32_t slots, cudaStream_t stream, uint32_t prop_block, uint32_t iters_per_graph, bool use_graph, bool host_paths = true);
     uint32_t slots() const { return slots_; }
     cudaStream_t stream() const { return stream_; }
     QueryParams& host_params(uint32_t slot) { return h_params_[slot]; }
@@ -79,6 +80,9 @@ class Engine {
     // and goal are taken from device memory instead of the host params.
     kgmt_status admit(uint32_t first, uint32_t count, uint32_t n_active, const float* d_inits = nullptr,
                       const float* d_goals = nullptr);
+    // admit(0, 1, 1) of a one-slot engine as one launch; the boxes come from
+    // p.raw_obstacles (device)
+    kgmt_status admit_only(const QueryParams& p);
     // the pieces of admit, for callers that admit several slot ranges
     kgmt_status upload_params(uint32_t first, uint32_t count);
     kgmt_status init_slots(uint32_t first, uint32_t count, const float* d_inits = nullptr, const float* d_goals = nullptr);
@@ -105,6 +109,13 @@ class Engine {
     // states and the error bits in one wait
     kgmt_status read_states_and_error(uint32_t first, uint32_t count, QueryState* out, uint32_t* err);
     kgmt_status extract_paths(uint32_t n_active);
+    // after run_until_done: the paths walked, the states of slots [0, count)
+    // and the error bits on the host, in one wait (none when the tail launch
+    // that ended the run already brought them)
+    kgmt_status finish(uint32_t count, QueryState* out, uint32_t* err);
+    // the rows of a state's path in the host path buffer (of the last finish;
+    // overwritten by the next run), or nullptr when they are on the device only
+    const float* host_path(const QueryState& s) const { return s.path_at == kNoPath || s.path_len == 0 ? nullptr : h_paths_ + s.path_at; }
     kgmt_status read_error(uint32_t* err);
     kgmt_status set_prop_block(uint32_t block);
     uint32_t prop_block() const { return prop_block_; }
@@ -166,7 +177,11 @@ class Engine {
     uint32_t* d_slot_list_ = nullptr;  // [slots] slots of a served admission
     uint32_t* h_running_ = nullptr;  // mapped pinned host words: [0] Sched::host_running, [1] error readback,
                                      // [2] tail iterations, [3] tail stopped for size
-    QueryState* h_stage_states_ = nullptr;  // pinned staging for state readbacks
+    QueryState* h_stage_states_ = nullptr;  // mapped pinned: states as k_paths or a readback leaves them, then the paths
+    const float* h_paths_ = nullptr;        // the paths' rows in that block
+    HostSink sink_ = {};                    // device addresses of the two
+    bool results_ready_ = false;  // the last run's states and paths are on the host
+    bool bar_zero_ = false;       // the tail launch's barrier is known to be zero
     uint32_t* d_running_ = nullptr;  // its device address
     cudaEvent_t ev_[2] = {nullptr, nullptr};
     cudaGraphExec_t graph_ = nullptr;

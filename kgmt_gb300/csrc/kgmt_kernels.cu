@@ -159,19 +159,11 @@ __device__ __forceinline__ void stage_box(const float* r, int w, float4* dst)
         }
 }
 
-// ---------------------------------------------------------------------------
-// admission: root node, cleared region tables, first frontier (root x5); the
-// slots are [first, first + count), or slots[0 .. count) when a list is given
-// ---------------------------------------------------------------------------
-__global__ void k_admit(const QueryParams* __restrict__ P, QueryState* S, uint32_t first, uint32_t count, const uint32_t* __restrict__ slots)
+// region tables and look-back words of a query at zero: this thread's share,
+// t of nt
+__device__ __forceinline__ void clear_tables(const QueryParams& p, uint32_t t, uint32_t nt)
 {
-    if(blockIdx.x >= count) return;
-    const uint32_t q = slots ? slots[blockIdx.x] : first + blockIdx.x;
-    const QueryParams& p = P[q];
-    if(p.raw_obstacles)
-        for(uint32_t o = threadIdx.x; o < p.n_obstacles; o += blockDim.x)
-            stage_box(p.raw_obstacles + (size_t)o * 2 * p.raw_w, p.raw_w, p.obstacles + 2 * o);
-    for(uint32_t r = threadIdx.x; r < p.regions; r += blockDim.x)
+    for(uint32_t r = t; r < p.regions; r += nt)
         {
             p.counter[r] = 0;
             p.valid[r] = 0;
@@ -179,11 +171,17 @@ __global__ void k_admit(const QueryParams* __restrict__ P, QueryState* S, uint32
             p.marks[r] = 0ull;
             p.newmarks[r] = 0ull;
         }
-    for(uint32_t i = threadIdx.x; i < p.tiles_per_chain; i += blockDim.x)
+    for(uint32_t i = t; i < p.tiles_per_chain; i += nt)
         {
             p.tiles_old[i] = 0ull;
             p.tiles_slot[i] = 0ull;
         }
+}
+
+// the root node, the first frontier (root x5) and the loop state of a query;
+// by one block
+__device__ __forceinline__ void admit_root(const QueryParams& p, QueryState& out)
+{
     for(uint32_t j = threadIdx.x; j < p.sample_dim; j += blockDim.x) p.tree[j] = p.init[j];
     if(threadIdx.x < kRootRepeat) p.rep_new[threadIdx.x] = 0u;
     if(threadIdx.x == 0)
@@ -201,10 +199,27 @@ __global__ void k_admit(const QueryParams* __restrict__ P, QueryState* S, uint32
             st.goal_index = -1;
             st.steps = 0;
             st.tests = 0;
+            st.path_at = kNoPath;
             st.t_start = globaltimer();
             plan_samples(p, st);
-            S[q] = st;
+            out = st;
         }
+}
+
+// ---------------------------------------------------------------------------
+// admission: root node, cleared region tables, first frontier (root x5); the
+// slots are [first, first + count), or slots[0 .. count) when a list is given
+// ---------------------------------------------------------------------------
+__global__ void k_admit(const QueryParams* __restrict__ P, QueryState* S, uint32_t first, uint32_t count, const uint32_t* __restrict__ slots)
+{
+    if(blockIdx.x >= count) return;
+    const uint32_t q = slots ? slots[blockIdx.x] : first + blockIdx.x;
+    const QueryParams& p = P[q];
+    if(p.raw_obstacles)
+        for(uint32_t o = threadIdx.x; o < p.n_obstacles; o += blockDim.x)
+            stage_box(p.raw_obstacles + (size_t)o * 2 * p.raw_w, p.raw_w, p.obstacles + 2 * o);
+    clear_tables(p, threadIdx.x, blockDim.x);
+    admit_root(p, S[q]);
 }
 
 // ---------------------------------------------------------------------------
@@ -322,6 +337,50 @@ __global__ void k_schedule(const QueryParams* __restrict__ P, const QueryState* 
                            uint32_t* tile_c_base, uint32_t* tile_c_old)
 {
     compute_schedule(P, S, sched, tile_a_base, tile_c_base, tile_c_old);
+}
+
+// Admission of an engine's only query: what k_stage_obstacles, the params
+// upload, k_set_n_slots, k_admit, k_build_grid, k_schedule and the barrier's
+// memset do in seven stream operations.  Block 0 takes the query (its build of
+// the grid is the longest part), the other blocks clear the region tables.  A
+// single plan's first iteration starts about 10 us after the call's first
+// launch instead of 45.
+__global__ void __launch_bounds__(256) k_begin(const __grid_constant__ QueryParams p, const LaunchArgs a, TailScratch* ts)
+{
+    __shared__ alignas(16) char mem[kGridBuildBytes];
+    __shared__ uint32_t scratch[34];
+    if(blockIdx.x > 0)
+        {
+            clear_tables(p, (blockIdx.x - 1) * blockDim.x + threadIdx.x, (gridDim.x - 1) * blockDim.x);
+            return;
+        }
+    QueryParams* dst = const_cast<QueryParams*>(a.params);
+    for(uint32_t i = threadIdx.x; i < sizeof(QueryParams) / 4; i += blockDim.x) ((uint32_t*)dst)[i] = ((const uint32_t*)&p)[i];
+    static_assert(sizeof(QueryParams) % 4 == 0 && sizeof(QueryState) % 8 == 0, "copied by words");
+    for(uint32_t o = threadIdx.x; o < p.n_obstacles; o += blockDim.x)
+        stage_box(p.raw_obstacles + (size_t)o * 2 * p.raw_w, p.raw_w, p.obstacles + 2 * o);
+    admit_root(p, a.states[0]);
+    if(threadIdx.x == 0)
+        {
+            a.sched->n_slots = 1;
+            a.sched->path_words = 0;
+            ts->bar = 0;
+        }
+    __syncthreads();
+    if(threadIdx.x == 0) dst->raw_obstacles = nullptr;  // the caller's array: not kept past this launch
+    if(p.grid_start != nullptr)
+        {
+            uint32_t total = 0;
+            const uint16_t* start = build_grid(p, p.obstacles, p.n_obstacles, p.grid_budget, mem, scratch, p.grid_items, &total);
+            if(start)
+                for(uint32_t c = threadIdx.x; c <= kGridCells; c += blockDim.x) p.grid_start[c] = start[c];
+            if(threadIdx.x == 0)
+                {
+                    p.grid_meta[0] = total;
+                    p.grid_meta[1] = start ? 1u : 0u;
+                }
+        }
+    compute_schedule(a.params, a.states, a.sched, a.tile_a_base, a.tile_c_base, a.tile_c_old);
 }
 
 template <int NT, int MODELS>
@@ -703,27 +762,77 @@ __global__ void __launch_bounds__(kAppendThreads, 8) k_append(const QueryParams*
 // ---------------------------------------------------------------------------
 // goal -> root path walk for finished queries (KGMT.cu:344-360)
 // ---------------------------------------------------------------------------
-__global__ void k_paths(const QueryParams* __restrict__ P, QueryState* S, uint32_t n)
+// One warp a query: lane 0 follows the parents (a chain of dependent loads,
+// ~0.4 us a node, and the only serial part), then all lanes copy the rows
+// together.  What the host reads goes straight to its pinned memory: the
+// states, the error bits and, packed one path behind the other, the rows of
+// every path found by this launch (paths longer than kPathChunk rows, or past
+// the buffer, stay on the device only).  A thread that walked and copied node
+// by node took ~1 us a node (22 us for 22 nodes; now 9).
+constexpr uint32_t kPathChunk = 128;  // nodes walked before their rows are copied
+constexpr int kPathWarps = 4;         // queries per block
+
+__global__ void __launch_bounds__(32 * kPathWarps) k_paths(const QueryParams* __restrict__ P, QueryState* S, uint32_t n, Sched* sched,
+                                                           const HostSink sink)
 {
-    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ int32_t s_node[kPathWarps][kPathChunk];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, q = blockIdx.x * kPathWarps + warp;
+    if(blockIdx.x == 0 && threadIdx.x == 0 && sink.error) *sink.error = sched->error;
     if(q >= n) return;
     QueryState& st = S[q];
-    if(st.status != KGMT_QUERY_SUCCESS || st.path_len != 0) return;
-    const QueryParams& p = P[q];
-    const uint32_t D = p.sample_dim;
-    const uint32_t max_rows = p.max_iterations + 2;
-    int32_t i = st.goal_index;
-    uint32_t len = 0;
-    while(i >= 0 && len < max_rows)
+    if(st.status == KGMT_QUERY_SUCCESS && st.path_len == 0)
         {
-            const float* src = p.tree + (size_t)i * D;
-            float* dst = p.path + (size_t)len * D;
-            for(uint32_t c = 0; c < D; ++c) dst[c] = src[c];
-            ++len;
-            i = p.parent[i];
+            const QueryParams& p = P[q];
+            const uint32_t D = p.sample_dim, max_rows = p.max_iterations + 2;
+            const float* tree = p.tree;
+            const int32_t* parent = p.parent;
+            const int32_t goal = st.goal_index;
+            int32_t i = goal;
+            uint32_t len = 0, at = kNoPath;
+            while(i >= 0 && len < max_rows)
+                {
+                    uint32_t k = 0;
+                    if(lane == 0)
+                        for(; k < kPathChunk && i >= 0 && len + k < max_rows; ++k)
+                            {
+                                s_node[warp][k] = i;
+                                i = __ldg(parent + i);
+                            }
+                    k = __shfl_sync(0xffffffffu, k, 0);
+                    i = __shfl_sync(0xffffffffu, i, 0);
+                    // the whole path is in hand: its place in the host buffer
+                    const bool whole = len == 0 && (i < 0 || k >= max_rows);
+                    if(whole && sink.paths)
+                        {
+                            if(lane == 0)
+                                {
+                                    at = atomicAdd(&sched->path_words, k * D);
+                                    if(at > sink.path_words || k * D > sink.path_words - at) at = kNoPath;
+                                }
+                            at = __shfl_sync(0xffffffffu, at, 0);
+                        }
+                    float* dev = p.path + (size_t)len * D;
+#pragma unroll 4
+                    for(uint32_t e = lane; e < k * D; e += 32)
+                        {
+                            const float v = __ldg(tree + (size_t)s_node[warp][e / D] * D + e % D);
+                            dev[e] = v;
+                            if(at != kNoPath) sink.paths[at + e] = v;
+                        }
+                    len += k;
+                    __syncwarp();
+                }
+            if(lane == 0)
+                {
+                    st.goal_cost = p.cost[goal];
+                    st.path_at = at;
+                    st.path_len = len;
+                }
+            __syncwarp();
         }
-    st.goal_cost = p.cost[st.goal_index];
-    st.path_len = len;
+    if(sink.states)
+        for(uint32_t j = lane; j < sizeof(QueryState) / 8; j += 32)
+            ((unsigned long long*)(sink.states + q))[j] = ((const unsigned long long*)&st)[j];
 }
 
 // ---------------------------------------------------------------------------
@@ -1023,10 +1132,19 @@ cudaError_t launch_schedule(const LaunchArgs& a, cudaStream_t s)
     return cudaGetLastError();
 }
 
-cudaError_t launch_paths(const LaunchArgs& a, uint32_t n, cudaStream_t s)
+cudaError_t launch_paths(const LaunchArgs& a, uint32_t n, const HostSink& sink, cudaStream_t s)
 {
     if(n == 0) return cudaSuccess;
-    k_paths<<<(n + 127) / 128, 128, 0, s>>>(a.params, a.states, n);
+    k_paths<<<(n + kPathWarps - 1) / kPathWarps, 32 * kPathWarps, 0, s>>>(a.params, a.states, n, a.sched, sink);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_begin(const LaunchArgs& a, const QueryParams& p, TailScratch* ts, cudaStream_t s)
+{
+    // four table entries a thread, up to four blocks' worth of threads per SM
+    const uint32_t items = p.regions > p.tiles_per_chain ? p.regions : p.tiles_per_chain;
+    const uint32_t clear = std::min<uint32_t>((items + 1023u) / 1024u, 608u);
+    k_begin<<<1 + clear, 256, 0, s>>>(p, a, ts);
     return cudaGetLastError();
 }
 
@@ -1090,13 +1208,16 @@ static cudaError_t launch_tail_t(const LaunchArgs& a, TailScratch* ts, int grid,
 }
 
 cudaError_t launch_tail(const LaunchArgs& a, TailScratch* ts, int models, int grid, uint32_t smem_boxes, uint32_t max_samples,
-                        uint32_t* host_words, cudaStream_t s)
+                        uint32_t* host_words, bool zero_bar, cudaStream_t s)
 {
     if(grid < 2 * kTailQueries || grid > kTailMaxBlocks) return cudaErrorInvalidValue;
     const uint32_t boxes = smem_boxes < kSmemBoxesMin ? kSmemBoxesMin : smem_boxes > (uint32_t)kSmemObstacles ? (uint32_t)kSmemObstacles : smem_boxes;
     // the barrier counter starts each launch at zero
-    cudaError_t e = cudaMemsetAsync(&ts->bar, 0, sizeof(uint32_t), s);
-    if(e != cudaSuccess) return e;
+    if(zero_bar)
+        {
+            const cudaError_t e = cudaMemsetAsync(&ts->bar, 0, sizeof(uint32_t), s);
+            if(e != cudaSuccess) return e;
+        }
     switch(models)
         {
             case kBitDI: return launch_tail_t<kBitDI>(a, ts, grid, boxes, max_samples, host_words, s);

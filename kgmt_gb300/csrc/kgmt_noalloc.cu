@@ -215,7 +215,7 @@ extern "C" kgmt_status kgmt_plan_noalloc(const kgmt_config* cfg, const float* h_
             NA_CHECK(cuda_status(cudaMemcpyAsync(&running, &d_sched->running, sizeof(uint32_t), cudaMemcpyDeviceToHost, s), "poll"));
             NA_CHECK(cuda_status(cudaStreamSynchronize(s), "cudaStreamSynchronize"));
         }
-    NA_CHECK(cuda_status(launch_paths(a, 1, s), "k_paths"));
+    NA_CHECK(cuda_status(launch_paths(a, 1, HostSink{}, s), "k_paths"));
     QueryState state;
     uint32_t err = 0;
     NA_CHECK(cuda_status(cudaMemcpyAsync(&state, d_state, sizeof(state), cudaMemcpyDeviceToHost, s), "download(state)"));

@@ -187,6 +187,8 @@ struct QueryState {
     uint32_t samples_drawn;
     uint32_t path_len;
     float goal_cost;      // the goal node's cost (set with the path)
+    uint32_t path_at;     // first word of the path's rows in the host path buffer (kNoPath: not there)
+    uint32_t pad;
     unsigned long long t_start;  // %globaltimer at admission (ns)
     unsigned long long t_end;
     unsigned long long steps;    // RK4 steps executed over all samples
@@ -212,9 +214,22 @@ struct Sched {
     // iteration's finalisers for the schedule of the next one
     unsigned long long next_samples;
     unsigned long long next_tree;
+    uint32_t path_words;  // words of the host path buffer handed out
+    uint32_t pad;
     // mapped pinned host word that mirrors `running` (or null): the host polls
     // it without a copy in the stream between graph replays
     uint32_t* host_running;
+};
+
+constexpr uint32_t kNoPath = 0xFFFFFFFFu;
+
+// Where k_paths leaves what the host reads after a plan, in mapped pinned
+// memory (no copies behind the kernel); null members: not wanted.
+struct HostSink {
+    QueryState* states;    // [n]
+    uint32_t* error;       // Sched::error
+    float* paths;          // the found paths' rows, packed
+    uint32_t path_words;   // capacity of paths, in floats
 };
 
 // device-side scratch of the persistent tail launch (kgmt_tail.cuh), one per engine
