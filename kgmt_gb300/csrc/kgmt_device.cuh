@@ -59,6 +59,19 @@ __device__ __forceinline__ float u01(uint32_t x) { return (float)((x >> 8) + 1u)
 // (oracle/fit_sincos.py).  Same operations as the CPU restatement, so both
 // round identically; accuracy about one ulp for |x| < 1e4.
 // ---------------------------------------------------------------------------
+// sine and cosine from those of the reduced argument: t, the reduction's sum,
+// holds the quadrant q in its two lowest bits.  Odd quadrants swap the two;
+// the sine is negative in quadrants 2 and 3 (bit 1 of q), the cosine in 1 and 2
+// (bit 1 of q + 1): sign-bit flips, the bits moved up by 30.
+__device__ __forceinline__ void quadrant(float t, float sp, float cp, float& s, float& c)
+{
+    const uint32_t q = __float_as_uint(t);
+    const float ss = (q & 1u) ? cp : sp;
+    const float cc = (q & 1u) ? sp : cp;
+    s = __uint_as_float(__float_as_uint(ss) ^ ((q << 30) & 0x80000000u));
+    c = __uint_as_float(__float_as_uint(cc) ^ ((q * 0x40000000u + 0x40000000u) & 0x80000000u));
+}
+
 __device__ __forceinline__ void sincos_portable(float x, float& s, float& c)
 {
     // explicit fused multiply-adds (one rounding each), placed exactly as in
@@ -71,7 +84,6 @@ __device__ __forceinline__ void sincos_portable(float x, float& s, float& c)
     // compute the same values.
     const float t = x * 0x1.45f306p-1f + 0x1.8p23f;
     const float n = t - 0x1.8p23f;
-    const int q = __float_as_int(t) & 3;
     float r = fmaf(-n, 0x1.92p+0f, x);
     r = fmaf(-n, 0x1.fb4p-12f, r);
     r = fmaf(-n, 0x1.4442d2p-24f, r);
@@ -83,11 +95,68 @@ __device__ __forceinline__ void sincos_portable(float x, float& s, float& c)
     pc = fmaf(r2, pc, 0x1.55554ap-5f);
     pc = fmaf(r2, pc, -0x1.0p-1f);
     float cp = fmaf(r2, pc, 1.0f);
-    float ss = (q & 1) ? cp : sp;
-    float cc = (q & 1) ? sp : cp;
-    // sine negative in quadrants 2 and 3, cosine in 1 and 2: sign-bit flips
-    s = __int_as_float(__float_as_int(ss) ^ ((q & 2) << 30));
-    c = __int_as_float(__float_as_int(cc) ^ (((q + 1) & 2) << 30));
+    quadrant(t, sp, cp, s, c);
+}
+
+// ---------------------------------------------------------------------------
+// Pairs of floats in one 64-bit register: sm_103a's packed fma / mul / add do
+// both halves in one instruction, each rounded on its own exactly as the scalar
+// operation.  The quadrotor is bound by instruction issue (78 % of the slots,
+// the FMA pipes 58 % busy), so a pair costs half.
+// ---------------------------------------------------------------------------
+struct F2 {
+    unsigned long long v;
+};
+
+__device__ __forceinline__ F2 pack2(float lo, float hi)
+{
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ F2 both(float x) { return pack2(x, x); }
+__device__ __forceinline__ void unpack2(F2 a, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v)); }
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b)
+{
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+
+// sincos_portable of both halves, the same operations
+__device__ __forceinline__ void sincos2(F2 x, float& s0, float& c0, float& s1, float& c1)
+{
+    const F2 t = add2(mul2(x, both(0x1.45f306p-1f)), both(0x1.8p23f));
+    const F2 n = add2(t, both(-0x1.8p23f));
+    F2 r = fma2(n, both(-0x1.92p+0f), x);
+    r = fma2(n, both(-0x1.fb4p-12f), r);
+    r = fma2(n, both(-0x1.4442d2p-24f), r);
+    const F2 r2 = mul2(r, r);
+    F2 ps = fma2(r2, both(-0x1.9943ep-13f), both(0x1.11073ap-7f));
+    ps = fma2(r2, ps, both(-0x1.555546p-3f));
+    const F2 sp = fma2(mul2(r, r2), ps, r);
+    F2 pc = fma2(r2, both(0x1.99eba6p-16f), both(-0x1.6c0c34p-10f));
+    pc = fma2(r2, pc, both(0x1.55554ap-5f));
+    pc = fma2(r2, pc, both(-0x1.0p-1f));
+    const F2 cp = fma2(r2, pc, both(1.0f));
+    float t0, t1, sp0, sp1, cp0, cp1;
+    unpack2(t, t0, t1);
+    unpack2(sp, sp0, sp1);
+    unpack2(cp, cp0, cp1);
+    quadrant(t0, sp0, cp0, s0, c0);
+    quadrant(t1, sp1, cp1, s1, c1);
 }
 
 // ---------------------------------------------------------------------------
@@ -561,36 +630,34 @@ __device__ __forceinline__ bool propagate_unicycle(const QueryParams& P, const G
 // [Zc Lc Mc Nc], classic RK4 over the rigid-body ode of
 // statePropagator.cu:325-370 (Euler-angle kinematics, drag -nu|v|, -mu|w|).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void quad_ode(const QueryParams& P, const float* s, float zc, float lc, float mc, float nc, float* d)
+// The state goes in pairs: (x y) (z psi) (phi theta) (u v) (w p) (q r).
+__device__ __forceinline__ void quad_ode(const QueryParams& P, const F2* s, float zc, float lc, float mc, float nc, F2* d)
 {
-    const float phi = s[3], theta = s[4], psi = s[5];
-    const float uu = s[6], vv = s[7], ww = s[8];
-    const float p = s[9], q = s[10], r = s[11];
+    float psi, uu, vv, ww, p, q, r, z;
+    unpack2(s[1], z, psi);
+    unpack2(s[3], uu, vv);
+    unpack2(s[4], ww, p);
+    unpack2(s[5], q, r);
     float sphi, cphi, sth, cth, spsi, cpsi;
-    sincos_portable(phi, sphi, cphi);
-    sincos_portable(theta, sth, cth);
+    sincos2(s[2], sphi, cphi, sth, cth);
     sincos_portable(psi, spsi, cpsi);
     // the two terms over cos(theta) share one division
     const float icth = 1.0f / cth;
     const float tth = sth * icth;
     const float g = P.gravity;
     const float sps = sphi * sth, cps = cphi * sth;
-    d[0] = fmaf(fmaf(cps, cpsi, sphi * spsi), ww, fmaf(fmaf(sps, cpsi, -(cphi * spsi)), vv, (cth * cpsi) * uu));
-    d[1] = fmaf(fmaf(cps, spsi, -(sphi * cpsi)), ww, fmaf(fmaf(sps, spsi, cphi * cpsi), vv, (cth * spsi) * uu));
-    d[2] = fmaf(cphi * cth, ww, fmaf(sphi * cth, vv, (-sth) * uu));
+    d[0] = pack2(fmaf(fmaf(cps, cpsi, sphi * spsi), ww, fmaf(fmaf(sps, cpsi, -(cphi * spsi)), vv, (cth * cpsi) * uu)),
+                 fmaf(fmaf(cps, spsi, -(sphi * cpsi)), ww, fmaf(fmaf(sps, spsi, cphi * cpsi), vv, (cth * spsi) * uu)));
     const float qr = fmaf(q, sphi, r * cphi);
-    d[3] = fmaf(qr, tth, p);
-    d[4] = fmaf(q, cphi, -(r * sphi));
-    d[5] = qr * icth;
+    d[1] = pack2(fmaf(cphi * cth, ww, fmaf(sphi * cth, vv, (-sth) * uu)), qr * icth);
+    d[2] = pack2(fmaf(qr, tth, p), fmaf(q, cphi, -(r * sphi)));
     const float xyz = (-P.nu) * sqrtf(fmaf(ww, ww, fmaf(vv, vv, uu * uu)));
     const float mx = P.mass_inv * xyz;
-    d[6] = fmaf(mx, uu, fmaf(-g, sth, fmaf(r, vv, -(q * ww))));
-    d[7] = fmaf(mx, vv, fmaf(g * cth, sphi, fmaf(p, ww, -(r * uu))));
-    d[8] = fmaf(P.mass_inv, zc, fmaf(mx, ww, fmaf(g * cth, cphi, fmaf(q, uu, -(p * vv)))));
+    d[3] = pack2(fmaf(mx, uu, fmaf(-g, sth, fmaf(r, vv, -(q * ww)))), fmaf(mx, vv, fmaf(g * cth, sphi, fmaf(p, ww, -(r * uu)))));
     const float lmn = (-P.mu) * sqrtf(fmaf(r, r, fmaf(q, q, p * p)));
-    d[9] = fmaf(P.iix, lc, fmaf(P.iix * lmn, p, (P.jx * q) * r));
-    d[10] = fmaf(P.iiy, mc, fmaf(P.iiy * lmn, q, (P.jy * p) * r));
-    d[11] = fmaf(P.iiz, nc, fmaf(P.iiz * lmn, r, (P.jz * p) * q));
+    d[4] = pack2(fmaf(P.mass_inv, zc, fmaf(mx, ww, fmaf(g * cth, cphi, fmaf(q, uu, -(p * vv))))),
+                 fmaf(P.iix, lc, fmaf(P.iix * lmn, p, (P.jx * q) * r)));
+    d[5] = pack2(fmaf(P.iiy, mc, fmaf(P.iiy * lmn, q, (P.jy * p) * r)), fmaf(P.iiz, nc, fmaf(P.iiz * lmn, r, (P.jz * p) * q)));
 }
 
 template <typename Grid>
@@ -606,44 +673,53 @@ __device__ __forceinline__ bool propagate_quad(const QueryParams& P, const Grid&
     // RK4 with the stage sum accumulated as each derivative arrives:
     // acc = k1; acc = fma(2, k2, acc); acc = fma(2, k3, acc); acc += k4 is
     // exactly fma(2, k3, fma(2, k2, k1)) + k4, with one derivative live at a time
-    float s[12], k[12], t[12], acc[12];
-#pragma unroll
-    for(int j = 0; j < 12; ++j) s[j] = x0[j];
-    StepCells sc = start_cells(P, s[0], s[1], s[2]);
+    F2 s[6] = {pack2(x0[0], x0[1]), pack2(x0[2], x0[5]), pack2(x0[3], x0[4]), pack2(x0[6], x0[7]), pack2(x0[8], x0[9]), pack2(x0[10], x0[11])};
+    F2 k[6], t[6], acc[6];
+    const F2 two = both(2.0f);
+    float px = x0[0], py = x0[1], pz = x0[2];
+    StepCells sc = start_cells(P, px, py, pz);
     bool ok = true;
     int done = 0;
     for(int i = 0; i < k_steps; ++i)
         {
             ++done;
-            const float q0 = s[0], q1 = s[1], q2 = s[2];
+            const float q0 = px, q1 = py, q2 = pz;
             quad_ode(P, s, zc, lc, mc, nc, k);
 #pragma unroll
-            for(int j = 0; j < 12; ++j) acc[j] = k[j], t[j] = fmaf(hh, k[j], s[j]);
+            for(int j = 0; j < 6; ++j) acc[j] = k[j], t[j] = fma2(both(hh), k[j], s[j]);
             quad_ode(P, t, zc, lc, mc, nc, k);
 #pragma unroll
-            for(int j = 0; j < 12; ++j) acc[j] = fmaf(2.0f, k[j], acc[j]), t[j] = fmaf(hh, k[j], s[j]);
+            for(int j = 0; j < 6; ++j) acc[j] = fma2(two, k[j], acc[j]), t[j] = fma2(both(hh), k[j], s[j]);
             quad_ode(P, t, zc, lc, mc, nc, k);
 #pragma unroll
-            for(int j = 0; j < 12; ++j) acc[j] = fmaf(2.0f, k[j], acc[j]), t[j] = fmaf(h, k[j], s[j]);
+            for(int j = 0; j < 6; ++j) acc[j] = fma2(two, k[j], acc[j]), t[j] = fma2(both(h), k[j], s[j]);
             quad_ode(P, t, zc, lc, mc, nc, k);
 #pragma unroll
-            for(int j = 0; j < 12; ++j) s[j] = fmaf(h6, acc[j] + k[j], s[j]);
-            const bool out = (s[6] < P.v_min) | (s[6] > P.v_max) | (s[7] < P.v_min) | (s[7] > P.v_max) | (s[8] < P.v_min) |
-                             (s[8] > P.v_max) | (s[0] < P.ws_min) | (s[0] > P.ws_max) | (s[1] < P.ws_min) | (s[1] > P.ws_max) |
-                             (s[2] < P.ws_min) | (s[2] > P.ws_max);
+            for(int j = 0; j < 6; ++j) s[j] = fma2(both(h6), add2(acc[j], k[j]), s[j]);
+            float psi, vx, vy, vz, p;
+            unpack2(s[0], px, py);
+            unpack2(s[1], pz, psi);
+            unpack2(s[3], vx, vy);
+            unpack2(s[4], vz, p);
+            const bool out = (vx < P.v_min) | (vx > P.v_max) | (vy < P.v_min) | (vy > P.v_max) | (vz < P.v_min) | (vz > P.v_max) |
+                             (px < P.ws_min) | (px > P.ws_max) | (py < P.ws_min) | (py > P.ws_max) | (pz < P.ws_min) | (pz > P.ws_max);
             if(out)
                 {
                     ok = false;
                     break;
                 }
-            if(!step_free(P, grid, obs, n_obs, q0, q1, q2, s[0], s[1], s[2], sc, cnt))
+            if(!step_free(P, grid, obs, n_obs, q0, q1, q2, px, py, pz, sc, cnt))
                 {
                     ok = false;
                     break;
                 }
         }
-#pragma unroll
-    for(int j = 0; j < 12; ++j) x1[j] = s[j];
+    unpack2(s[0], x1[0], x1[1]);
+    unpack2(s[1], x1[2], x1[5]);
+    unpack2(s[2], x1[3], x1[4]);
+    unpack2(s[3], x1[6], x1[7]);
+    unpack2(s[4], x1[8], x1[9]);
+    unpack2(s[5], x1[10], x1[11]);
     x1[12] = zc, x1[13] = lc, x1[14] = mc, x1[15] = nc;
     x1[16] = h * (float)k_steps;
     cnt.steps = done;
