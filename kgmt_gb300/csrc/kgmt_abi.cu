@@ -206,6 +206,7 @@ static kgmt_status plan_setup(kgmt_planner* p, const float* h_initial, const flo
     p->params.raw_w = (int32_t)ws_dims_of(p->cfg.model);
     p->eng.set_models(Engine::model_bit(p->cfg.model));
     p->eng.set_max_obstacles(n_obstacles);
+    p->eng.set_large_tables(p->params.regions > kScoreSmall);
     const kgmt_status st = p->eng.admit_only(p->params);
     p->params.raw_obstacles = nullptr;  // the caller's array
     return st;
@@ -425,7 +426,7 @@ static kgmt_status batch_prepare(kgmt_batch* b, uint32_t n, const kgmt_config* c
     RETURN_IF(!cfgs || !obs_offset || !obs_count, KGMT_ERR_INVALID_ARG, "batch: NULL argument");
     b->eng.reset_counters();
     uint64_t boxes = 0;
-    uint32_t max_iters = 0, max_obs = 0;
+    uint32_t max_iters = 0, max_obs = 0, max_regions = 0;
     size_t total = 0;
     std::vector<QueryLayout> L(n);
     for(uint32_t i = 0; i < n; ++i)
@@ -437,6 +438,7 @@ static kgmt_status batch_prepare(kgmt_batch* b, uint32_t n, const kgmt_config* c
             if(end > boxes) boxes = end;
             if(obs_count[i] > max_obs) max_obs = obs_count[i];
             if(cfgs[i].max_iterations > max_iters) max_iters = cfgs[i].max_iterations;
+            max_regions = std::max(max_regions, regions_of(cfgs[i]));
         }
     RETURN_IF(boxes > (1ull << 31), KGMT_ERR_INVALID_ARG, "batch: too many obstacles");
     const size_t obs_bytes = ((boxes * 32 + 255) / 256) * 256;
@@ -451,6 +453,7 @@ static kgmt_status batch_prepare(kgmt_batch* b, uint32_t n, const kgmt_config* c
     for(uint32_t i = 0; i < n; ++i) models |= Engine::model_bit(cfgs[i].model);
     b->eng.set_models(models);
     b->eng.set_max_obstacles(max_obs);
+    b->eng.set_large_tables(max_regions > kScoreSmall);
     b->params.resize(n);
     for(uint32_t i = 0; i < n; ++i)
         {
@@ -727,6 +730,7 @@ struct kgmt_server {
     uint64_t next_ticket = 1;
     uint32_t resident = 0;     // admitted and not yet retired
     uint32_t box_capacity = 0; // boxes a propagate block stages: the largest admitted so far
+    uint32_t max_regions = 0;  // the largest region table admitted so far
     bool resched = false;      // a resident query was cancelled: the next step recomputes the schedule
     // the step in flight: its iterations and the copy of states [0, copied)
     bool inflight = false;
@@ -881,6 +885,7 @@ extern "C" kgmt_status kgmt_server_step(kgmt_server* s, uint32_t* n_running, uin
             r.offset = off;
             r.submitted = q.submitted;
             if(n_obs > s->box_capacity) s->box_capacity = n_obs;
+            s->max_regions = std::max(s->max_regions, prm.regions);
             ++s->resident;
             ++slot;
         }
@@ -908,6 +913,7 @@ extern "C" kgmt_status kgmt_server_step(kgmt_server* s, uint32_t* n_running, uin
                 if(s->slots[i].used) models |= s->slots[i].model_bit;
             s->eng.set_models(models);
             s->eng.set_max_obstacles(s->box_capacity);
+            s->eng.set_large_tables(s->max_regions > kScoreSmall);
             CHECK_ST(s->eng.schedule());
             s->resched = false;
         }

@@ -474,6 +474,7 @@ kgmt_status Engine::set_prop_block(uint32_t block)
     int dev = 0, sms = 0;
     KGMT_CUDA(cudaGetDevice(&dev), "cudaGetDevice");
     KGMT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
+    sms_ = sms;
     for(int m : {1, 2, 4, 8, 15}) grid_a_[m] = sms * propagate_blocks_per_sm((int)block, m);
     grid_c_ = sms * append_blocks_per_sm();
     // the tail launch: one block per SM (all blocks resident for its grid-wide
@@ -509,6 +510,17 @@ void Engine::set_max_obstacles(uint32_t max_obs)
     const uint32_t boxes = smem_boxes_for(max_obs);
     if(boxes == smem_boxes_) return;
     smem_boxes_ = boxes;
+    if(graph_)
+        {
+            cudaGraphExecDestroy(graph_);
+            graph_ = nullptr;
+        }
+}
+
+void Engine::set_large_tables(bool large)
+{
+    if(large == large_tables_) return;
+    large_tables_ = large;
     if(graph_)
         {
             cudaGraphExecDestroy(graph_);
@@ -627,7 +639,7 @@ kgmt_status Engine::record_event(cudaEvent_t* out)
 kgmt_status Engine::launch_iteration()
 {
     const LaunchArgs a = args();
-    // kernel kinds in the profile: 0 propagate (with the region scores), 2 append
+    // kernel kinds in the profile: 0 propagate (with the region scores and k_score), 2 append
     for(int k = 0; k < 3; k += 2)
         {
             if(profile_)
@@ -636,7 +648,11 @@ kgmt_status Engine::launch_iteration()
                     if(st != KGMT_OK) return st;
                     prof_kind_.push_back(k);
                 }
-            if(k == 0) KGMT_CUDA(launch_propagate(a, (int)prop_block_, models_, grid_a_[models_], smem_boxes_, stream_), "k_propagate");
+            if(k == 0)
+                {
+                    KGMT_CUDA(launch_propagate(a, (int)prop_block_, models_, grid_a_[models_], smem_boxes_, stream_), "k_propagate");
+                    if(large_tables_) KGMT_CUDA(launch_score(a, sms_, stream_), "k_score");
+                }
             else KGMT_CUDA(launch_append(a, grid_c_, stream_), "k_append");
             if(profile_)
                 {
@@ -644,7 +660,7 @@ kgmt_status Engine::launch_iteration()
                     if(st != KGMT_OK) return st;
                 }
         }
-    launches_ += 2;
+    launches_ += large_tables_ ? 3 : 2;
     return KGMT_OK;
 }
 
@@ -746,7 +762,7 @@ kgmt_status Engine::launch_unit()
                     if(st != KGMT_OK) return st;
                 }
             KGMT_CUDA(cudaGraphLaunch(graph_, stream_), "cudaGraphLaunch");
-            launches_ += 2ull * iters_per_graph_;
+            launches_ += (large_tables_ ? 3ull : 2ull) * iters_per_graph_;
         }
     else
         {

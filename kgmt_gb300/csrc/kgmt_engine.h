@@ -61,6 +61,7 @@ QueryLayout layout_of(const kgmt_config& c, uint32_t n_obstacles, bool inline_ob
 QueryParams make_params(const kgmt_config& c, const float* init, const float* goal, char* chunk, const QueryLayout& L, float4* obstacles,
                         uint32_t n_obstacles);
 uint32_t sample_dim_of(int32_t model);
+uint32_t regions_of(const kgmt_config& c);
 uint32_t ws_dims_of(int32_t model);
 kgmt_result to_result(const QueryState& s, uint64_t ticket);
 
@@ -127,6 +128,9 @@ class Engine {
     // largest box count of the admitted queries: sizes the propagate kernel's
     // shared-memory box stage (a change drops the graph)
     void set_max_obstacles(uint32_t max_obs);
+    // whether an admitted query may have more than kScoreSmall regions: the
+    // chain then has a k_score launch (a change drops the graph)
+    void set_large_tables(bool large);
     static int model_bit(int32_t model)
     {
         return model == KGMT_MODEL_QUADROTOR ? 2 : model == KGMT_MODEL_DUBINS_AIRPLANE ? 4 : model == KGMT_MODEL_UNICYCLE ? 8 : 1;
@@ -166,6 +170,8 @@ class Engine {
     bool use_graph_ = true;
     int grid_a_[16] = {};           // propagate grid per variant
     int grid_c_ = 0;
+    int sms_ = 0;
+    bool large_tables_ = true;      // the chain scores large region tables in their own launch
     int models_ = 15;               // propagate variant (Engine::variant_of)
     uint32_t smem_boxes_ = kSmemObstacles;  // boxes staged in shared memory per propagate block
     QueryParams* d_params_ = nullptr;

@@ -735,63 +735,40 @@ struct ScoreParams
     float epsilon, cell_volume;
 };
 
-template <int NT>
-__device__ void update_scores(const ScoreParams& p, QueryState& st, float* lanes)
+__device__ __forceinline__ ScoreParams score_params(const QueryParams& p)
 {
-    const float F = (float)p.fine_cells;
-    constexpr int U = 4;  // regions whose loads are issued together
-    // the thread's first U regions keep their raw score in registers for the
-    // normalisation pass (no re-read of what it just wrote)
-    float kept[U];
-    for(int l = threadIdx.x; l < kScoreLanes; l += NT)
-        {
-            float acc = 0.0f;
-            for(uint32_t r0 = (uint32_t)l; r0 < p.regions; r0 += U * kScoreLanes)
-                {
-                    const bool first = l == (int)threadIdx.x && r0 == (uint32_t)l;
-                    uint64_t m[U];
-                    int32_t nv[U], n[U];
-#pragma unroll
-                    for(int k = 0; k < U; ++k)
-                        {
-                            const uint32_t r = r0 + k * kScoreLanes;
-                            if(r < p.regions)
-                                {
-                                    m[k] = __ldcg(&p.marks[r]) | __ldcg(&p.newmarks[r]);
-                                    nv[k] = __ldcg(&p.valid[r]);
-                                    n[k] = __ldcg(&p.counter[r]);
-                                }
-                        }
-                    // regions in increasing order: the lane's sum keeps its fixed order
-#pragma unroll
-                    for(int k = 0; k < U; ++k)
-                        {
-                            const uint32_t r = r0 + k * kScoreLanes;
-                            if(r >= p.regions) break;
-                            p.marks[r] = m[k];
-                            p.newmarks[r] = 0ull;
-                            float raw = 0.0f;    // adds nothing to the total
-                            float keep = -1.0f;  // marks "no valid sample" for the normalisation pass
-                            if(nv[k] > 0)
-                                {
-                                    const float cov = (float)__popcll(m[k]) / F;
-                                    const float a = p.epsilon + (float)nv[k];
-                                    const float b = a + (float)(n[k] - nv[k]);
-                                    const float fv = (a / b) * p.cell_volume;
-                                    const float f2 = fv * fv;
-                                    const float f4 = f2 * f2;
-                                    const float nf = (float)n[k];
-                                    const float den = (1.0f + cov) * (1.0f + nf * nf);
-                                    raw = f4 / den;
-                                    keep = raw;
-                                }
-                            p.score[r] = keep;
-                            if(first) kept[k] = keep;
-                            acc = acc + raw;
-                        }
-                }
-            lanes[l] = acc;
-        }
+    return {p.counter, p.valid, p.score, p.marks, p.newmarks, p.regions, p.fine_cells, p.epsilon, p.cell_volume};
+}
+
+// raw score of a region with n samples, nv of them valid, and the visited fine
+// cells m; -1 marks "no valid sample" for the normalisation
+__device__ __forceinline__ float raw_score(const ScoreParams& p, float F, uint64_t m, int32_t nv, int32_t n)
+{
+    if(nv <= 0) return -1.0f;
+    const float cov = (float)__popcll(m) / F;
+    const float a = p.epsilon + (float)nv;
+    const float b = a + (float)(n - nv);
+    const float fv = (a / b) * p.cell_volume;
+    const float f2 = fv * fv;
+    const float f4 = f2 * f2;
+    const float nf = (float)n;
+    const float den = (1.0f + cov) * (1.0f + nf * nf);
+    return f4 / den;
+}
+
+// what a raw score adds to the total
+__device__ __forceinline__ float scored(float raw) { return raw < 0.0f ? 0.0f : raw; }
+
+// raw score (-1 for regions without valid samples) -> normalised score
+__device__ __forceinline__ float norm_score(const ScoreParams& p, float raw, float total)
+{
+    return raw < 0.0f ? 1.0f : (total > 0.0f ? p.epsilon + raw / total : p.epsilon);
+}
+
+// halving tree over the lanes' sums; every thread gets the total.  Block-uniform.
+template <int NT>
+__device__ __forceinline__ float lanes_total(float* lanes)
+{
     __syncthreads();
     static_assert(kScoreLanes >= 64, "the last five halving levels run in one warp");
     for(int stride = kScoreLanes / 2; stride >= 32; stride >>= 1)
@@ -809,10 +786,48 @@ __device__ void update_scores(const ScoreParams& p, QueryState& st, float* lanes
             if(threadIdx.x == 0) lanes[0] = v;
         }
     __syncthreads();
-    const float total = lanes[0];
-    // raw score (-1 for regions without valid samples) -> normalised score;
-    // past the registers each lane re-reads only what it wrote itself
-    auto norm = [&](float raw) { return raw < 0.0f ? 1.0f : (total > 0.0f ? p.epsilon + raw / total : p.epsilon); };
+    return lanes[0];
+}
+
+// a table of at most kScoreSmall regions, by one block
+template <int NT>
+__device__ void update_scores(const ScoreParams& p, QueryState& st, float* lanes)
+{
+    const float F = (float)p.fine_cells;
+    constexpr int U = (int)kScoreSmall / kScoreLanes;  // a lane's regions: loaded together, their raw scores kept in registers
+    float kept[U];
+    for(int l = threadIdx.x; l < kScoreLanes; l += NT)
+        {
+            uint64_t m[U];
+            int32_t nv[U], n[U];
+#pragma unroll
+            for(int k = 0; k < U; ++k)
+                {
+                    const uint32_t r = (uint32_t)l + k * kScoreLanes;
+                    if(r < p.regions)
+                        {
+                            m[k] = __ldcg(&p.marks[r]) | __ldcg(&p.newmarks[r]);
+                            nv[k] = __ldcg(&p.valid[r]);
+                            n[k] = __ldcg(&p.counter[r]);
+                        }
+                }
+            // regions in increasing order: the lane's sum keeps its fixed order
+            float acc = 0.0f;
+#pragma unroll
+            for(int k = 0; k < U; ++k)
+                {
+                    const uint32_t r = (uint32_t)l + k * kScoreLanes;
+                    if(r >= p.regions) break;
+                    p.marks[r] = m[k];
+                    p.newmarks[r] = 0ull;
+                    const float raw = raw_score(p, F, m[k], nv[k], n[k]);
+                    if(l == (int)threadIdx.x) kept[k] = raw;
+                    else p.score[r] = raw;
+                    acc = acc + scored(raw);
+                }
+            lanes[l] = acc;
+        }
+    const float total = lanes_total<NT>(lanes);
     for(int l = threadIdx.x; l < kScoreLanes; l += NT)
         {
             uint32_t r = (uint32_t)l;
@@ -820,9 +835,90 @@ __device__ void update_scores(const ScoreParams& p, QueryState& st, float* lanes
                 {
 #pragma unroll
                     for(int k = 0; k < U; ++k, r += kScoreLanes)
-                        if(r < p.regions) p.score[r] = norm(kept[k]);
+                        if(r < p.regions) p.score[r] = norm_score(p, kept[k], total);
                 }
-            for(; r < p.regions; r += kScoreLanes) p.score[r] = norm(p.score[r]);
+            // more lanes than threads: the rest re-reads what it wrote itself
+            for(; r < p.regions; r += kScoreLanes) p.score[r] = norm_score(p, p.score[r], total);
+        }
+    if(threadIdx.x == 0) st.score_total = total;
+}
+
+// Slice `slice` of a larger table: its raw scores into the table, the
+// iteration's new cells into the marks.  Four consecutive regions a thread and
+// round, their counters in 16-byte loads (the tables start 256-byte aligned).
+template <int NT>
+__device__ __forceinline__ void score_slice(const ScoreParams& p, uint32_t slice)
+{
+    const float F = (float)p.fine_cells;
+    const uint32_t end = min(p.regions, (slice + 1u) * kScoreSlice);
+    for(uint32_t r = slice * kScoreSlice + threadIdx.x * 4u; r < end; r += NT * 4u)
+        {
+            if(r + 3 < end)
+                {
+                    const ulonglong2 ma = __ldcg((const ulonglong2*)(p.marks + r)), mb = __ldcg((const ulonglong2*)(p.marks + r) + 1);
+                    const ulonglong2 wa = __ldcg((const ulonglong2*)(p.newmarks + r)), wb = __ldcg((const ulonglong2*)(p.newmarks + r) + 1);
+                    const int4 nv = __ldcg((const int4*)(p.valid + r)), n = __ldcg((const int4*)(p.counter + r));
+                    if(wa.x | wa.y | wb.x | wb.y)
+                        {
+                            *(ulonglong2*)(p.marks + r) = make_ulonglong2(ma.x | wa.x, ma.y | wa.y);
+                            *((ulonglong2*)(p.marks + r) + 1) = make_ulonglong2(mb.x | wb.x, mb.y | wb.y);
+                            *(ulonglong2*)(p.newmarks + r) = make_ulonglong2(0ull, 0ull);
+                            *((ulonglong2*)(p.newmarks + r) + 1) = make_ulonglong2(0ull, 0ull);
+                        }
+                    *(float4*)(p.score + r) = make_float4(raw_score(p, F, ma.x | wa.x, nv.x, n.x), raw_score(p, F, ma.y | wa.y, nv.y, n.y),
+                                                          raw_score(p, F, mb.x | wb.x, nv.z, n.z), raw_score(p, F, mb.y | wb.y, nv.w, n.w));
+                }
+            else
+                for(uint32_t j = r; j < end; ++j)
+                    {
+                        const uint64_t m = __ldcg(&p.marks[j]) | __ldcg(&p.newmarks[j]);
+                        p.marks[j] = m;
+                        p.newmarks[j] = 0ull;
+                        p.score[j] = raw_score(p, F, m, __ldcg(&p.valid[j]), __ldcg(&p.counter[j]));
+                    }
+        }
+}
+
+// total and normalisation of a table whose slices are all scored (by other
+// blocks: read past L1), by one block
+template <int NT>
+__device__ __forceinline__ void score_finish(const ScoreParams& p, QueryState& st, float* lanes)
+{
+    constexpr int U = 16;  // loads in flight a thread
+    for(int l = threadIdx.x; l < kScoreLanes; l += NT)
+        {
+            // regions l, l + 256, ... in order
+            float acc = 0.0f;
+            uint32_t r = (uint32_t)l;
+            for(; r + (U - 1) * kScoreLanes < p.regions; r += U * kScoreLanes)
+                {
+                    float v[U];
+#pragma unroll
+                    for(int k = 0; k < U; ++k) v[k] = __ldcg(p.score + r + k * kScoreLanes);
+#pragma unroll
+                    for(int k = 0; k < U; ++k) acc = acc + scored(v[k]);
+                }
+            for(; r < p.regions; r += kScoreLanes) acc = acc + scored(__ldcg(p.score + r));
+            lanes[l] = acc;
+        }
+    const float total = lanes_total<NT>(lanes);
+    constexpr int V = 4;  // 16-byte loads in flight a thread
+    for(uint32_t r0 = threadIdx.x * 4u; r0 < p.regions; r0 += V * NT * 4u)
+        {
+            float4 v[V];
+#pragma unroll
+            for(int k = 0; k < V; ++k)
+                if(r0 + k * NT * 4u + 3u < p.regions) v[k] = __ldcg((const float4*)(p.score + r0 + k * NT * 4u));
+#pragma unroll
+            for(int k = 0; k < V; ++k)
+                {
+                    const uint32_t r = r0 + k * NT * 4u;
+                    if(r + 3u < p.regions)
+                        *(float4*)(p.score + r) = make_float4(norm_score(p, v[k].x, total), norm_score(p, v[k].y, total),
+                                                              norm_score(p, v[k].z, total), norm_score(p, v[k].w, total));
+                    else
+                        for(uint32_t j = r; j < p.regions; ++j) p.score[j] = norm_score(p, __ldcg(p.score + j), total);
+                }
         }
     if(threadIdx.x == 0) st.score_total = total;
 }

@@ -509,15 +509,70 @@ __global__ void __launch_bounds__(NT, (MODELS == kBitDI ? 1024 : 512) / NT) k_pr
                     s_tile = (int)t;
                 }
             __syncthreads();
-            if(s_last)
+            if(s_last && s_p.regions <= kScoreSmall)
                 {
                     __threadfence();
-                    const ScoreParams sp{s_p.counter, s_p.valid, s_p.score, s_p.marks, s_p.newmarks, s_p.regions, s_p.fine_cells, s_p.epsilon, s_p.cell_volume};
-                    update_scores<NT>(sp, S[q], s_lanes);
+                    update_scores<NT>(score_params(s_p), S[q], s_lanes);
                 }
             t = (uint32_t)s_tile;
             __syncthreads();
         }
+}
+
+// Region scores of the queries with large tables, between the propagate and the
+// append launch (only in chains that hold such a query).  The slices of all of
+// them go round the blocks; the block that finishes a query's last slice sums
+// and normalises, so no block ever waits for another.
+constexpr int kScoreThreads = 256;
+constexpr int kScoreBlocksPerSm = 3;
+
+__global__ void __launch_bounds__(kScoreThreads, kScoreBlocksPerSm) k_score(const QueryParams* __restrict__ P, QueryState* S,
+                                                                           const Sched* sched)
+{
+    __shared__ uint32_t scratch[34];
+    __shared__ uint32_t s_pre[kScoreThreads + 1];  // first slice of each slot of the group
+    __shared__ float s_lanes[kScoreLanes];
+    __shared__ int s_last;
+    // the slices are counted from the append kernel's schedule, complete before
+    // the propagate kernel let this one start; what that one counts is read
+    // only past the wait (which every block reaches)
+    pdl_trigger();
+    const uint32_t n_slots = sched->n_slots;
+    bool waited = false;
+    uint32_t before = 0;  // slices of earlier groups of slots
+    for(uint32_t c0 = 0; c0 < n_slots; c0 += kScoreThreads)
+        {
+            const uint32_t i = c0 + threadIdx.x;
+            uint32_t slices = 0;
+            if(i < n_slots && S[i].status == KGMT_QUERY_RUNNING && S[i].n_samples > 0 && P[i].regions > kScoreSmall)
+                slices = (P[i].regions + kScoreSlice - 1) / kScoreSlice;
+            uint32_t total;
+            s_pre[threadIdx.x] = block_exclusive_scan<kScoreThreads>(slices, scratch, &total);
+            if(threadIdx.x == 0) s_pre[kScoreThreads] = total;
+            if(!waited) pdl_wait();
+            waited = true;
+            __syncthreads();
+            for(uint32_t j = (blockIdx.x + gridDim.x - before % gridDim.x) % gridDim.x; j < total; j += gridDim.x)
+                {
+                    const int g = find_slot(s_pre, kScoreThreads, j);
+                    const uint32_t q = c0 + (uint32_t)g;
+                    const ScoreParams sp = score_params(P[q]);
+                    QueryState& st = S[q];
+                    score_slice<kScoreThreads>(sp, j - s_pre[g]);
+                    __syncthreads();
+                    if(threadIdx.x == 0) s_last = atomic_add_release(&st.score_done, 1u) == s_pre[g + 1] - s_pre[g] - 1u;
+                    __syncthreads();
+                    if(s_last)
+                        {
+                            __threadfence();
+                            if(threadIdx.x == 0) st.score_done = 0;
+                            score_finish<kScoreThreads>(sp, st, s_lanes);
+                        }
+                }
+            before += total;
+            __syncthreads();
+        }
+    if(!waited) pdl_wait();
 }
 
 // eight blocks per SM (32 registers; the kernel waits on loads, scans and
@@ -1114,6 +1169,13 @@ cudaError_t launch_append(const LaunchArgs& a, int grid, cudaStream_t s)
     cudaLaunchAttribute attr[1];
     const cudaLaunchConfig_t cfg = dependent_config(grid, kAppendThreads, 0, s, attr);
     return cudaLaunchKernelEx(&cfg, k_append, a.params, a.states, a.sched, a.tile_a_base, a.tile_c_base, a.tile_c_old);
+}
+
+cudaError_t launch_score(const LaunchArgs& a, int sms, cudaStream_t s)
+{
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = dependent_config(sms * kScoreBlocksPerSm, kScoreThreads, 0, s, attr);
+    return cudaLaunchKernelEx(&cfg, k_score, a.params, a.states, (const Sched*)a.sched);
 }
 
 cudaError_t launch_admit(const LaunchArgs& a, uint32_t first, uint32_t count, cudaStream_t s, const uint32_t* slots)

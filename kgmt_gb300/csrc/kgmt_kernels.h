@@ -22,6 +22,9 @@ cudaError_t launch_schedule(const LaunchArgs& a, cudaStream_t s);
 // smem_boxes: boxes a block stages in shared memory (the largest query of the
 // launch, rounded by smem_boxes_for); more are read from global memory
 cudaError_t launch_propagate(const LaunchArgs& a, int block, int models, int grid, uint32_t smem_boxes, cudaStream_t s);
+// region scores of queries with more than kScoreSmall regions (between propagate
+// and append; needed when the launch may meet such a query)
+cudaError_t launch_score(const LaunchArgs& a, int sms, cudaStream_t s);
 cudaError_t launch_append(const LaunchArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_paths(const LaunchArgs& a, uint32_t n, const HostSink& sink, cudaStream_t s);
 // admission of the engine's only query in one launch: its params (by value,

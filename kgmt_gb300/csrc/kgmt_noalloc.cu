@@ -210,6 +210,7 @@ extern "C" kgmt_status kgmt_plan_noalloc(const kgmt_config* cfg, const float* h_
             for(int k = 0; k < 4; ++k)
                 {
                     NA_CHECK(cuda_status(launch_propagate(a, (int)block, models, grid_a, smem_boxes_for(n_obstacles), s), "k_propagate"));
+                    if(params.regions > kScoreSmall) NA_CHECK(cuda_status(launch_score(a, sms, s), "k_score"));
                     NA_CHECK(cuda_status(launch_append(a, grid_c, s), "k_append"));
                 }
             NA_CHECK(cuda_status(cudaMemcpyAsync(&running, &d_sched->running, sizeof(uint32_t), cudaMemcpyDeviceToHost, s), "poll"));

@@ -122,6 +122,7 @@ __device__ __forceinline__ void thread_items(uint32_t n, uint32_t parts, uint32_
 struct TailQuery {
     int slot;
     uint32_t status, itr, tree, n_react, w_new, spe, n_samples, drawn;
+    uint32_t slices;  // of a large region table (0: scored by one block)
     uint32_t react_total, acc_total, w_total, n_next;
     float fa;
 };
@@ -203,6 +204,8 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
             Q.spe = __ldcg(&st.spe);
             Q.n_samples = __ldcg(&st.n_samples);
             Q.drawn = __ldcg(&st.samples_drawn);
+            const uint32_t regions = P[Q.slot].regions;
+            Q.slices = regions > kScoreSmall ? (regions + kScoreSlice - 1) / kScoreSlice : 0u;
         }
     if(b == 0 && threadIdx.x < 2 * kTailQueries)
         {
@@ -220,11 +223,11 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
             // ---- the iteration's size; the running queries split the blocks
             // into contiguous ranges (a block keeps its query and its staged
             // boxes until a query finishes) ----
-            uint32_t tot = 0;
+            uint32_t tot = 0, large = 0;
             int nr = 0, rq[kTailQueries];
 #pragma unroll
             for(int q = 0; q < kTailQueries; ++q)
-                if(q < nq && tq[q].status == KGMT_QUERY_RUNNING) tot += tq[q].n_samples, rq[nr++] = q;
+                if(q < nq && tq[q].status == KGMT_QUERY_RUNNING) tot += tq[q].n_samples, large += tq[q].slices, rq[nr++] = q;
             if(nr == 0) break;
             if(tot > max_samples)
                 {
@@ -330,10 +333,8 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                 {
                     if(tq[b].status == KGMT_QUERY_RUNNING)
                         {
-                            const QueryParams& gp = P[tq[b].slot];
-                            const ScoreParams sp{gp.counter, gp.valid, gp.score, gp.marks, gp.newmarks, gp.regions, gp.fine_cells, gp.epsilon,
-                                                 gp.cell_volume};
-                            update_scores<NT>(sp, S[tq[b].slot], s_lanes);
+                            const ScoreParams sp = score_params(P[tq[b].slot]);
+                            if(sp.regions <= kScoreSmall) update_scores<NT>(sp, S[tq[b].slot], s_lanes);
                         }
                 }
             else
@@ -368,6 +369,24 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                                 ts->rep_cnt[q][b - nq] = v[1];
                             }
                     }
+            // slices of large region tables go round the blocks (from the last
+            // one down, so that few fall to the blocks that scored a small one);
+            // once all are scored, one block a query sums and normalises
+            if(large)
+                {
+                    uint32_t before = 0;
+#pragma unroll 1
+                    for(int q = 0; q < nq; ++q)
+                        if(tq[q].status == KGMT_QUERY_RUNNING && tq[q].slices)
+                            {
+                                for(uint32_t j = (G - 1u - b + G - before % G) % G; j < tq[q].slices; j += G)
+                                    score_slice<NT>(score_params(P[tq[q].slot]), j);
+                                before += tq[q].slices;
+                            }
+                    if(!grid_barrier(&ts->bar, target, &sched->error)) return;
+                    if((int)b < nq && tq[b].status == KGMT_QUERY_RUNNING && tq[b].slices)
+                        score_finish<NT>(score_params(P[tq[b].slot]), S[tq[b].slot], s_lanes);
+                }
             if(b == 0 && threadIdx.x < kTailQueries)
                 {
                     // the other parity's copies start the next iteration from
