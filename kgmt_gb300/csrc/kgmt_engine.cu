@@ -444,8 +444,8 @@ kgmt_status Engine::init(uint32_t slots, cudaStream_t stream, uint32_t prop_bloc
     }
     // the running count and the tail launch's report, written by the device
     // into mapped pinned memory
-    KGMT_CUDA(cudaHostAlloc((void**)&h_running_, sizeof(uint32_t) * 4, cudaHostAllocMapped), "cudaHostAlloc(mapped)");
-    std::memset(h_running_, 0, sizeof(uint32_t) * 4);
+    KGMT_CUDA(cudaHostAlloc((void**)&h_running_, sizeof(uint32_t) * 8, cudaHostAllocMapped), "cudaHostAlloc(mapped)");
+    std::memset(h_running_, 0, sizeof(uint32_t) * 8);
     KGMT_CUDA(cudaHostGetDevicePointer((void**)&d_running_, h_running_, 0), "cudaHostGetDevicePointer");
     // the states and, packed, the rows of the paths found, as k_paths leaves
     // them: one pinned block (2 KiB of path a slot: 50 rows of the double
@@ -616,9 +616,8 @@ kgmt_status Engine::admit_only(const QueryParams& p)
     h_params_[0] = p;
     h_params_[0].raw_obstacles = nullptr;
     n_active_ = 1;
-    KGMT_CUDA(launch_begin(args(), p, d_tail_, stream_), "k_begin");
+    KGMT_CUDA(launch_begin(args(), p, stream_), "k_begin");
     launches_ += 1;
-    bar_zero_ = true;
     return KGMT_OK;
 }
 
@@ -694,9 +693,11 @@ kgmt_status Engine::run_tail(bool* done, bool* declined_at_once)
             if(st != KGMT_OK) return st;
             prof_kind_.push_back(1);
         }
-    KGMT_CUDA(launch_tail(args(), d_tail_, models_, tail_grid_[models_], smem_boxes_, tail_max_samples_, d_running_ + 2, !bar_zero_, stream_),
+    volatile uint32_t* w = h_running_;
+    w[2] = 0xFFFFFFFFu;  // a launch that gives up at a meeting point leaves it
+    // tags of 2^17 iterations a launch: more than max_iterations allows
+    KGMT_CUDA(launch_tail(args(), d_tail_, models_, tail_grid_[models_], smem_boxes_, tail_max_samples_, tail_seq_ << 17, d_running_ + 2, stream_),
               "k_tail");
-    bar_zero_ = false;
     if(profile_)
         {
             kgmt_status st = record_event(nullptr);
@@ -708,9 +709,13 @@ kgmt_status Engine::run_tail(bool* done, bool* declined_at_once)
     // running are left alone)
     kgmt_status ps = extract_paths(n_active_);
     if(ps != KGMT_OK) return ps;
-    KGMT_CUDA(cudaStreamSynchronize(stream_), "cudaStreamSynchronize");
-    volatile uint32_t* w = h_running_;
-    tail_iters_ += w[2];
+    const cudaError_t e = cudaStreamSynchronize(stream_);
+    // a launch that stopped at once left no tags behind
+    if(w[2] != 0u) ++tail_seq_;
+    KGMT_CUDA(e, "cudaStreamSynchronize");
+    if(w[2] != 0xFFFFFFFFu) tail_iters_ += w[2];
+    // its arrivals are unknown: the next launch starts from none
+    else KGMT_CUDA(cudaMemsetAsync(&d_tail_->arrivals, 0, 2 * sizeof(uint32_t), stream_), "memset(tail)");
     *done = w[0] == 0u;
     results_ready_ = *done;
     *declined_at_once = w[3] != 0u && w[2] == 0u;
@@ -782,7 +787,8 @@ kgmt_status Engine::run_until_done(uint32_t max_iters)
     // running count the last schedule wrote (unit u-1's or a later one's) is
     // read from the mapped host word; nothing but the event record sits in
     // the stream between two graph replays.  Once at most kTailQueries
-    // queries run, one persistent tail launch takes the iterations left (it
+    // queries run and their iteration is small enough (the schedule leaves its
+    // samples beside the count), one persistent tail launch takes the rest (it
     // hands back to the units when an iteration outgrows it; after a launch
     // that could not take even one iteration, the next attempt waits twice as
     // many units).
@@ -812,7 +818,7 @@ kgmt_status Engine::run_until_done(uint32_t max_iters)
                     const uint32_t n = *running;
                     if(n == 0) break;
                     if(wait_units > 0) --wait_units;
-                    else if(tail && n <= (uint32_t)kTailQueries)
+                    else if(tail && n <= (uint32_t)kTailQueries && running[4] <= tail_max_samples_)
                         {
                             bool done = false, at_once = false;
                             st = run_tail(&done, &at_once);

@@ -182,12 +182,12 @@ class Engine {
     uint32_t* d_tile_old_ = nullptr;
     uint32_t* d_slot_list_ = nullptr;  // [slots] slots of a served admission
     uint32_t* h_running_ = nullptr;  // mapped pinned host words: [0] Sched::host_running, [1] error readback,
-                                     // [2] tail iterations, [3] tail stopped for size
+                                     // [2] tail iterations, [3] tail stopped for size, [4] samples of the next iteration
     QueryState* h_stage_states_ = nullptr;  // mapped pinned: states as k_paths or a readback leaves them, then the paths
     const float* h_paths_ = nullptr;        // the paths' rows in that block
     HostSink sink_ = {};                    // device addresses of the two
     bool results_ready_ = false;  // the last run's states and paths are on the host
-    bool bar_zero_ = false;       // the tail launch's barrier is known to be zero
+    uint32_t tail_seq_ = 1;       // numbers the tail launches that ran iterations (their tags)
     uint32_t* d_running_ = nullptr;  // its device address
     cudaEvent_t ev_[2] = {nullptr, nullptr};
     cudaGraphExec_t graph_ = nullptr;

@@ -261,7 +261,7 @@ __device__ void compute_schedule(const QueryParams* __restrict__ P, const QueryS
     // totals only steer the tile sizes (thresholds below 2^22): clamped so
     // that no sum can wrap
     constexpr uint32_t kClamp = 1u << 22;
-    auto publish = [&](uint32_t tiles_a, uint32_t tiles_c, uint32_t running, uint32_t prop_tile, uint32_t old_tile) {
+    auto publish = [&](uint32_t tiles_a, uint32_t tiles_c, uint32_t running, uint32_t prop_tile, uint32_t old_tile, uint32_t samples) {
         tile_a_base[n] = tiles_a;
         tile_c_base[n] = tiles_c;
         sched->tiles_a = tiles_a;
@@ -273,7 +273,11 @@ __device__ void compute_schedule(const QueryParams* __restrict__ P, const QueryS
         sched->next_samples = 0ull;
         sched->next_tree = 0ull;
         if(running) sched->iterations += 1;
-        if(sched->host_running) *(volatile uint32_t*)sched->host_running = running;
+        if(sched->host_running)
+            {
+                *(volatile uint32_t*)(sched->host_running + 4) = samples;
+                *(volatile uint32_t*)sched->host_running = running;
+            }
     };
     if(n <= 32)
         {
@@ -310,7 +314,7 @@ __device__ void compute_schedule(const QueryParams* __restrict__ P, const QueryS
                             tile_c_base[q] = ic - tc;
                             tile_c_old[q] = told;
                         }
-                    if(q == 31) publish(ia, ic, ir, prop_tile, old_tile);
+                    if(q == 31) publish(ia, ic, ir, prop_tile, old_tile, tot_s);
                 }
             __syncthreads();
             return;
@@ -365,7 +369,7 @@ __device__ void compute_schedule(const QueryParams* __restrict__ P, const QueryS
                 }
             carry.x += sum.x, carry.y += sum.y, carry.z += sum.z;
         }
-    if(threadIdx.x == 0) publish(carry.x, carry.y, carry.z, prop_tile, old_tile);
+    if(threadIdx.x == 0) publish(carry.x, carry.y, carry.z, prop_tile, old_tile, tot.x);
     __syncthreads();
 }
 
@@ -529,9 +533,12 @@ __device__ __forceinline__ uint32_t prepare_sample(const QueryParams& p, const P
     return par;
 }
 
+// row, parent and word: where the sample's end row and parent go if it joins the
+// tree, and its region with the accept flag (global arrays, or shared memory)
 template <int MODEL>
 __device__ __forceinline__ void finish_sample(const QueryParams& p, const GridView& grid, const float4* obs, uint32_t n_obs, uint32_t s,
-                                              bool live, uint32_t par, const float* x0, const float* u, PropShared* sh)
+                                              bool live, uint32_t par, const float* x0, const float* u, PropShared* sh, float* row,
+                                              int32_t* parent, uint32_t* word)
 {
     constexpr int D = ModelDims<MODEL>::D;
     constexpr int NC = ModelDims<MODEL>::NC;
@@ -560,10 +567,10 @@ __device__ __forceinline__ void finish_sample(const QueryParams& p, const GridVi
             // flag, in one word (region ids are below 2^31)
             if(acc)
                 {
-                    store_row<D>(p.us + (size_t)s * D, x1);
-                    p.up[s] = (int32_t)par;
+                    store_row<D>(row, x1);
+                    *parent = (int32_t)par;
                 }
-            if(live) p.ur1f[s] = (uint32_t)r1 | (acc ? 0x80000000u : 0u);
+            if(live) *word = (uint32_t)r1 | (acc ? 0x80000000u : 0u);
         }
     // histogram updates (KGMT.cu:250-253): counter over all samples, valid
     // count and the fine-cell bit over the valid ones; one fire-and-forget L2
@@ -686,7 +693,10 @@ __device__ __forceinline__ void propagate_tile(const QueryParams& sp, const Prop
                     waited = true;
                 }
             const GridView grid{(sp.grid_meta != nullptr && s_gmeta[1] == 1u) ? s_gstart : nullptr, s_gitems, sp.grid_items};
-            with_model<MODELS>(model, [&](auto m) { finish_sample<decltype(m)::value>(sp, grid, obs, sp.n_obstacles, s, live, par, x0, u, sh); });
+            with_model<MODELS>(model, [&](auto m) {
+                constexpr int M = decltype(m)::value;
+                finish_sample<M>(sp, grid, obs, sp.n_obstacles, s, live, par, x0, u, sh, sp.us + (size_t)s * ModelDims<M>::D, sp.up + s, sp.ur1f + s);
+            });
         }
     // a thread that got no run still follows the copy's phase
     if(!waited) wait();
@@ -696,16 +706,17 @@ __device__ __forceinline__ void propagate_tile(const QueryParams& sp, const Prop
 // order -- no sort: with one such range per block the time of a launch is its
 // slowest warp's, which ordering the samples inside a block cannot shorten.
 // Parent rows are read coherently (they may have been appended by other
-// blocks in the same launch).  `wait` runs once, after the parents and draws
-// are gathered.  Block-uniform call.
+// blocks in the same launch); sample s0 + i leaves its end row, parent and
+// region word at rows + i D, parents + i and words + i.  `wait` runs once,
+// after the parents and draws are gathered.  Block-uniform call.
 template <int NT, int MODELS, typename Wait>
 __device__ __forceinline__ void propagate_range(const QueryParams& sp, const PropCtx& sc, uint32_t s0, uint32_t n, uint32_t smem_boxes,
                                                 PropShared* sh, const float4* s_obs, const uint16_t* s_gstart, const uint16_t* s_gitems,
-                                                const uint32_t* s_gmeta, Wait&& wait)
+                                                const uint32_t* s_gmeta, float* rows, int32_t* parents, uint32_t* words, Wait&& wait)
 {
     const int model = sp.model;
-    const uint32_t s = s0 + threadIdx.x;
-    const bool live = threadIdx.x < n && s < sc.n_samples;
+    const uint32_t i = threadIdx.x, s = s0 + i;
+    const bool live = i < n && s < sc.n_samples;
     float x0[KGMT_MAX_SAMPLE_DIM], u[8];
     uint32_t par = 0;
     if(live)
@@ -716,7 +727,10 @@ __device__ __forceinline__ void propagate_range(const QueryParams& sp, const Pro
     wait();
     const float4* obs = sp.n_obstacles <= smem_boxes ? s_obs : sp.obstacles;
     const GridView grid{(sp.grid_meta != nullptr && s_gmeta[1] == 1u) ? s_gstart : nullptr, s_gitems, sp.grid_items};
-    with_model<MODELS>(model, [&](auto m) { finish_sample<decltype(m)::value>(sp, grid, obs, sp.n_obstacles, s, live, par, x0, u, sh); });
+    with_model<MODELS>(model, [&](auto m) {
+        constexpr int M = decltype(m)::value;
+        finish_sample<M>(sp, grid, obs, sp.n_obstacles, s, live, par, x0, u, sh, rows + (size_t)i * ModelDims<M>::D, parents + i, words + i);
+    });
 }
 
 // Graph::updateVertices (Graph.cu:311-358) for one query, by one block: all
@@ -765,25 +779,27 @@ __device__ __forceinline__ float norm_score(const ScoreParams& p, float raw, flo
     return raw < 0.0f ? 1.0f : (total > 0.0f ? p.epsilon + raw / total : p.epsilon);
 }
 
-// halving tree over the lanes' sums; every thread gets the total.  Block-uniform.
-template <int NT>
+// halving tree over the lanes' sums (lane l adds lane l + stride, strides 128 ..
+// 1); every thread gets the total.  Block-uniform.  One warp does all levels in
+// registers: thread t holds lanes t, t + 32, ..., so the strides of 32 and more
+// stay inside it and the rest are shuffles -- no block barrier a level.
 __device__ __forceinline__ float lanes_total(float* lanes)
 {
     __syncthreads();
-    static_assert(kScoreLanes >= 64, "the last five halving levels run in one warp");
-    for(int stride = kScoreLanes / 2; stride >= 32; stride >>= 1)
-        {
-            for(int l = threadIdx.x; l < stride; l += NT) lanes[l] = lanes[l] + lanes[l + stride];
-            __syncthreads();
-        }
     if(threadIdx.x < 32)
         {
-            // strides 16 .. 1 in registers: lane l < stride adds lane l + stride,
-            // the same additions in the same order as the levels above
-            float v = lanes[threadIdx.x];
+            constexpr int K = kScoreLanes / 32;
+            static_assert((K & (K - 1)) == 0, "halving levels");
+            float v[K];
 #pragma unroll
-            for(int stride = 16; stride >= 1; stride >>= 1) v = v + __shfl_down_sync(0xffffffffu, v, stride);
-            if(threadIdx.x == 0) lanes[0] = v;
+            for(int k = 0; k < K; ++k) v[k] = lanes[threadIdx.x + 32 * k];
+#pragma unroll
+            for(int h = K / 2; h >= 1; h >>= 1)
+#pragma unroll
+                for(int k = 0; k < h; ++k) v[k] = v[k] + v[k + h];
+#pragma unroll
+            for(int stride = 16; stride >= 1; stride >>= 1) v[0] = v[0] + __shfl_down_sync(0xffffffffu, v[0], stride);
+            if(threadIdx.x == 0) lanes[0] = v[0];
         }
     __syncthreads();
     return lanes[0];
@@ -827,7 +843,7 @@ __device__ void update_scores(const ScoreParams& p, QueryState& st, float* lanes
                 }
             lanes[l] = acc;
         }
-    const float total = lanes_total<NT>(lanes);
+    const float total = lanes_total(lanes);
     for(int l = threadIdx.x; l < kScoreLanes; l += NT)
         {
             uint32_t r = (uint32_t)l;
@@ -901,7 +917,7 @@ __device__ __forceinline__ void score_finish(const ScoreParams& p, QueryState& s
             for(; r < p.regions; r += kScoreLanes) acc = acc + scored(__ldcg(p.score + r));
             lanes[l] = acc;
         }
-    const float total = lanes_total<NT>(lanes);
+    const float total = lanes_total(lanes);
     constexpr int V = 4;  // 16-byte loads in flight a thread
     for(uint32_t r0 = threadIdx.x * 4u; r0 < p.regions; r0 += V * NT * 4u)
         {
@@ -1003,10 +1019,10 @@ __device__ __forceinline__ float append_row(const QueryParams& p, const float* s
 }
 
 // KGMT.cu:387-388
-__device__ __forceinline__ float f_accept_vals(const QueryParams& p, uint32_t tree_size, uint32_t n_next, uint32_t itr)
+__device__ __forceinline__ float f_accept_vals(uint32_t capacity, float epsilon, uint32_t tree_size, uint32_t n_next, uint32_t itr)
 {
-    const float ta = 1.0f - (float)(tree_size + n_next) / (float)p.capacity;
-    const float ie = (float)itr * p.epsilon;
+    const float ta = 1.0f - (float)(tree_size + n_next) / (float)capacity;
+    const float ie = (float)itr * epsilon;
     const double t = (double)ta;
     const double t5 = ((t * t) * (t * t)) * t;
     return (float)((double)ie * t5);
@@ -1014,7 +1030,7 @@ __device__ __forceinline__ float f_accept_vals(const QueryParams& p, uint32_t tr
 
 __device__ __forceinline__ float f_accept_of(const QueryParams& p, const QueryState& st)
 {
-    return f_accept_vals(p, st.tree_size, st.n_next, st.itr);
+    return f_accept_vals(p.capacity, p.epsilon, st.tree_size, st.n_next, st.itr);
 }
 
 

@@ -340,12 +340,12 @@ __global__ void k_schedule(const QueryParams* __restrict__ P, const QueryState* 
 }
 
 // Admission of an engine's only query: what k_stage_obstacles, the params
-// upload, k_set_n_slots, k_admit, k_build_grid, k_schedule and the barrier's
-// memset do in seven stream operations.  Block 0 takes the query (its build of
+// upload, k_set_n_slots, k_admit, k_build_grid and k_schedule do in six stream
+// operations.  Block 0 takes the query (its build of
 // the grid is the longest part), the other blocks clear the region tables.  A
 // single plan's first iteration starts about 10 us after the call's first
 // launch instead of 45.
-__global__ void __launch_bounds__(256) k_begin(const __grid_constant__ QueryParams p, const LaunchArgs a, TailScratch* ts)
+__global__ void __launch_bounds__(256) k_begin(const __grid_constant__ QueryParams p, const LaunchArgs a)
 {
     __shared__ alignas(16) char mem[kGridBuildBytes];
     __shared__ uint32_t scratch[34];
@@ -364,7 +364,6 @@ __global__ void __launch_bounds__(256) k_begin(const __grid_constant__ QueryPara
         {
             a.sched->n_slots = 1;
             a.sched->path_words = 0;
-            ts->bar = 0;
         }
     __syncthreads();
     if(threadIdx.x == 0) dst->raw_obstacles = nullptr;  // the caller's array: not kept past this launch
@@ -1201,12 +1200,12 @@ cudaError_t launch_paths(const LaunchArgs& a, uint32_t n, const HostSink& sink, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_begin(const LaunchArgs& a, const QueryParams& p, TailScratch* ts, cudaStream_t s)
+cudaError_t launch_begin(const LaunchArgs& a, const QueryParams& p, cudaStream_t s)
 {
     // four table entries a thread, up to four blocks' worth of threads per SM
     const uint32_t items = p.regions > p.tiles_per_chain ? p.regions : p.tiles_per_chain;
     const uint32_t clear = std::min<uint32_t>((items + 1023u) / 1024u, 608u);
-    k_begin<<<1 + clear, 256, 0, s>>>(p, a, ts);
+    k_begin<<<1 + clear, 256, 0, s>>>(p, a);
     return cudaGetLastError();
 }
 
@@ -1226,12 +1225,13 @@ template <int MODELS>
 static int tail_occupancy_t()
 {
     int n = 0;
-    if(cudaFuncSetAttribute(k_tail<MODELS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPropSmemBytes) != cudaSuccess)
+    const size_t smem = tail_smem_bytes(kSmemObstacles, tail_row_dim<MODELS>());
+    if(cudaFuncSetAttribute(k_tail<MODELS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         {
             cudaGetLastError();
             return 0;
         }
-    if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_tail<MODELS>, kTailThreads, kPropSmemBytes) != cudaSuccess)
+    if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_tail<MODELS>, kTailThreads, smem) != cudaSuccess)
         {
             cudaGetLastError();
             return 0;
@@ -1252,8 +1252,8 @@ int tail_blocks_per_sm(int models)
 }
 
 template <int MODELS>
-static cudaError_t launch_tail_t(const LaunchArgs& a, TailScratch* ts, int grid, uint32_t boxes, uint32_t max_samples, uint32_t* host_words,
-                                 cudaStream_t s)
+static cudaError_t launch_tail_t(const LaunchArgs& a, TailScratch* ts, int grid, uint32_t boxes, uint32_t max_samples, uint32_t tag0,
+                                 uint32_t* host_words, cudaStream_t s)
 {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -1261,32 +1261,26 @@ static cudaError_t launch_tail_t(const LaunchArgs& a, TailScratch* ts, int grid,
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid, 1, 1);
     cfg.blockDim = dim3((unsigned)kTailThreads, 1, 1);
-    cfg.dynamicSmemBytes = prop_smem_bytes(boxes);
+    cfg.dynamicSmemBytes = tail_smem_bytes(boxes, tail_row_dim<MODELS>());
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k_tail<MODELS>, a.params, a.states, a.sched, ts, a.tile_a_base, a.tile_c_base, a.tile_c_old, boxes,
-                              max_samples, host_words);
+                              max_samples, tag0, host_words);
 }
 
-cudaError_t launch_tail(const LaunchArgs& a, TailScratch* ts, int models, int grid, uint32_t smem_boxes, uint32_t max_samples,
-                        uint32_t* host_words, bool zero_bar, cudaStream_t s)
+cudaError_t launch_tail(const LaunchArgs& a, TailScratch* ts, int models, int grid, uint32_t smem_boxes, uint32_t max_samples, uint32_t tag0,
+                        uint32_t* host_words, cudaStream_t s)
 {
     if(grid < 2 * kTailQueries || grid > kTailMaxBlocks) return cudaErrorInvalidValue;
     const uint32_t boxes = smem_boxes < kSmemBoxesMin ? kSmemBoxesMin : smem_boxes > (uint32_t)kSmemObstacles ? (uint32_t)kSmemObstacles : smem_boxes;
-    // the barrier counter starts each launch at zero
-    if(zero_bar)
-        {
-            const cudaError_t e = cudaMemsetAsync(&ts->bar, 0, sizeof(uint32_t), s);
-            if(e != cudaSuccess) return e;
-        }
     switch(models)
         {
-            case kBitDI: return launch_tail_t<kBitDI>(a, ts, grid, boxes, max_samples, host_words, s);
-            case kBitQuad: return launch_tail_t<kBitQuad>(a, ts, grid, boxes, max_samples, host_words, s);
-            case kBitDubins: return launch_tail_t<kBitDubins>(a, ts, grid, boxes, max_samples, host_words, s);
-            case kBitUnicycle: return launch_tail_t<kBitUnicycle>(a, ts, grid, boxes, max_samples, host_words, s);
-            default: return launch_tail_t<kAllModels>(a, ts, grid, boxes, max_samples, host_words, s);
+            case kBitDI: return launch_tail_t<kBitDI>(a, ts, grid, boxes, max_samples, tag0, host_words, s);
+            case kBitQuad: return launch_tail_t<kBitQuad>(a, ts, grid, boxes, max_samples, tag0, host_words, s);
+            case kBitDubins: return launch_tail_t<kBitDubins>(a, ts, grid, boxes, max_samples, tag0, host_words, s);
+            case kBitUnicycle: return launch_tail_t<kBitUnicycle>(a, ts, grid, boxes, max_samples, tag0, host_words, s);
+            default: return launch_tail_t<kAllModels>(a, ts, grid, boxes, max_samples, tag0, host_words, s);
         }
 }
 

@@ -29,8 +29,8 @@ cudaError_t launch_append(const LaunchArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_paths(const LaunchArgs& a, uint32_t n, const HostSink& sink, cudaStream_t s);
 // admission of the engine's only query in one launch: its params (by value,
 // written to slot 0), boxes (p.raw_obstacles), culling grid, region tables,
-// root, the first schedule, and the tail launch's barrier at zero
-cudaError_t launch_begin(const LaunchArgs& a, const QueryParams& p, TailScratch* ts, cudaStream_t s);
+// root and the first schedule
+cudaError_t launch_begin(const LaunchArgs& a, const QueryParams& p, cudaStream_t s);
 // src: rows of 2 * ws_dims floats (min corner, max corner)
 cudaError_t launch_stage_obstacles(const float* src, float4* dst, uint32_t n, int ws_dims, cudaStream_t s);
 // KGMT_CHECK_BOUNDS builds: the index-check error bits since the last call
@@ -50,8 +50,9 @@ int append_blocks_per_sm();
 size_t tail_scratch_bytes();
 // blocks of the tail kernel one SM holds (0: it cannot run)
 int tail_blocks_per_sm(int models);
-// zero_bar: the barrier counter is not known to be zero (it is after launch_begin)
-cudaError_t launch_tail(const LaunchArgs& a, TailScratch* ts, int models, int grid, uint32_t smem_boxes, uint32_t max_samples,
-                        uint32_t* host_words, bool zero_bar, cudaStream_t s);
+// tag0: the launch's meeting points are tagged tag0 + 1, ..., one an iteration;
+// no launch since the last one that ran an iteration may have used them
+cudaError_t launch_tail(const LaunchArgs& a, TailScratch* ts, int models, int grid, uint32_t smem_boxes, uint32_t max_samples, uint32_t tag0,
+                        uint32_t* host_words, cudaStream_t s);
 
 }  // namespace kgmt

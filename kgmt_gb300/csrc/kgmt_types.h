@@ -53,11 +53,15 @@ constexpr uint32_t kSpinLimit = 1u << 22;  // polls before a device-side wait gi
 
 constexpr uint32_t kSlotEmpty = 0xFFFFFFFFu;  // QueryState::status of a never-admitted slot
 
-// persistent tail launch (kgmt_tail.cuh): at most this many running queries,
-// one block of kTailThreads per SM, at most kTailMaxBlocks blocks
-constexpr int kTailQueries = 4;
+// persistent tail launch (kgmt_tail.cuh): at most this many running queries
+// (one a lane of the warp that divides the blocks among them), one block of
+// kTailThreads per SM, at most kTailShare samples a block and iteration.  (Four
+// queries before: a batch left with 5 to 32 running ones stayed in the chain at
+// 37 us an iteration and more.)
+constexpr int kTailQueries = 32;
 constexpr int kTailThreads = 256;
-constexpr int kTailMaxBlocks = 1024;
+constexpr int kTailMaxBlocks = kTailThreads;  // one exchange word a thread
+constexpr uint32_t kTailShare = 640;
 
 // static FP32 lane-operation counts per RK4 step, from the code in
 // kgmt_device.cuh (a multiply, add, fused multiply-add, divide or compare is
@@ -224,8 +228,9 @@ struct Sched {
     unsigned long long next_tree;
     uint32_t path_words;  // words of the host path buffer handed out
     uint32_t pad;
-    // mapped pinned host word that mirrors `running` (or null): the host polls
-    // it without a copy in the stream between graph replays
+    // mapped pinned host words (or null) that the host polls without a copy in
+    // the stream between graph replays: [0] mirrors `running`, [4] the samples
+    // of the next iteration (clamped to 2^22)
     uint32_t* host_running;
 };
 
@@ -241,18 +246,17 @@ struct HostSink {
 };
 
 // device-side scratch of the persistent tail launch (kgmt_tail.cuh), one per engine
+using TailBox = unsigned long long;  // iteration tag and payload of one block for another
 struct TailScratch {
-    uint32_t bar;         // grid-barrier arrivals of the running launch (zeroed before it)
     uint32_t iterations;  // iterations the last launch ran
     uint32_t declined;    // 1: the last launch stopped before an iteration larger than it takes
-    uint32_t pad;
     unsigned long long fp32_ops;  // algorithmic FP32 operations of the tail's propagation (host-zeroed)
     unsigned long long samples;   // samples the tail propagated (host-zeroed)
-    uint32_t n_next[2][kTailQueries];                 // accepted samples per query, by iteration parity
-    uint32_t goal[2][kTailQueries];                   // smallest new goal-ball index per query (~0u: none)
-    uint32_t old_cnt[kTailQueries][kTailMaxBlocks];   // re-activated nodes of each block's chunk
-    uint32_t acc_cnt[kTailQueries][kTailMaxBlocks];   // accepted samples of each block's chunk
-    uint32_t rep_cnt[kTailQueries][kTailMaxBlocks];   // frontier entries (repeats) of each block's chunk
+    uint32_t arrivals;    // blocks' arrivals at meeting points, ever growing
+    uint32_t arrived;     // what they were when the last launch ended
+    uint32_t word[kTailMaxBlocks];                // payload of each block's last arrival
+    TailBox box[kTailMaxBlocks][kTailMaxBlocks];  // [to][from]
+    uint32_t scored[kTailQueries];               // iteration tag: the query's region scores are ready
 };
 
 }  // namespace kgmt
