@@ -659,7 +659,7 @@ kgmt_status Engine::launch_iteration()
                     if(st != KGMT_OK) return st;
                 }
         }
-    launches_ += large_tables_ ? 3 : 2;
+    launches_ += large_tables_ ? 4 : 2;
     return KGMT_OK;
 }
 
@@ -767,7 +767,7 @@ kgmt_status Engine::launch_unit()
                     if(st != KGMT_OK) return st;
                 }
             KGMT_CUDA(cudaGraphLaunch(graph_, stream_), "cudaGraphLaunch");
-            launches_ += (large_tables_ ? 3ull : 2ull) * iters_per_graph_;
+            launches_ += (large_tables_ ? 4ull : 2ull) * iters_per_graph_;
         }
     else
         {

@@ -900,7 +900,7 @@ __device__ __forceinline__ void score_slice(const ScoreParams& p, uint32_t slice
 template <int NT>
 __device__ __forceinline__ void score_finish(const ScoreParams& p, QueryState& st, float* lanes)
 {
-    constexpr int U = 16;  // loads in flight a thread
+    constexpr int U = 32;  // loads in flight a thread
     for(int l = threadIdx.x; l < kScoreLanes; l += NT)
         {
             // regions l, l + 256, ... in order
@@ -918,7 +918,7 @@ __device__ __forceinline__ void score_finish(const ScoreParams& p, QueryState& s
             lanes[l] = acc;
         }
     const float total = lanes_total(lanes);
-    constexpr int V = 4;  // 16-byte loads in flight a thread
+    constexpr int V = 8;  // 16-byte loads in flight a thread
     for(uint32_t r0 = threadIdx.x * 4u; r0 < p.regions; r0 += V * NT * 4u)
         {
             float4 v[V];

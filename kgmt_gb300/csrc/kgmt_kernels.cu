@@ -519,22 +519,30 @@ __global__ void __launch_bounds__(NT, (MODELS == kBitDI ? 1024 : 512) / NT) k_pr
 }
 
 // Region scores of the queries with large tables, between the propagate and the
-// append launch (only in chains that hold such a query).  The slices of all of
-// them go round the blocks; the block that finishes a query's last slice sums
-// and normalises, so no block ever waits for another.
+// append launch (only in chains that hold such a query): k_score, raw scores,
+// the slices of all queries round the blocks; k_score_sum, total and
+// normalisation, one block a query.  Bound by L2 and DRAM latency.  As one launch
+// in which the block that finished a query's last slice summed it, 190 queries of
+// up to 32^3 regions took 75 us (some blocks summed three of them), now 27 + 16.
 constexpr int kScoreThreads = 256;
-constexpr int kScoreBlocksPerSm = 3;
+constexpr int kScoreBlocksPerSm = 6;
+constexpr int kSumThreads = 512;
+constexpr int kSumBlocksPerSm = 2;
 
-__global__ void __launch_bounds__(kScoreThreads, kScoreBlocksPerSm) k_score(const QueryParams* __restrict__ P, QueryState* S,
+// whether slot i has a large table to score in this iteration (the schedule's
+// values, complete before the propagate kernel let this launch start)
+__device__ __forceinline__ bool has_large_table(const QueryParams* P, const QueryState* S, uint32_t i)
+{
+    return S[i].status == KGMT_QUERY_RUNNING && S[i].n_samples > 0 && P[i].regions > kScoreSmall;
+}
+
+__global__ void __launch_bounds__(kScoreThreads, kScoreBlocksPerSm) k_score(const QueryParams* __restrict__ P, const QueryState* S,
                                                                            const Sched* sched)
 {
     __shared__ uint32_t scratch[34];
     __shared__ uint32_t s_pre[kScoreThreads + 1];  // first slice of each slot of the group
-    __shared__ float s_lanes[kScoreLanes];
-    __shared__ int s_last;
-    // the slices are counted from the append kernel's schedule, complete before
-    // the propagate kernel let this one start; what that one counts is read
-    // only past the wait (which every block reaches)
+    // what the propagate kernel counts is read only past the wait (which every
+    // block reaches)
     pdl_trigger();
     const uint32_t n_slots = sched->n_slots;
     bool waited = false;
@@ -542,9 +550,7 @@ __global__ void __launch_bounds__(kScoreThreads, kScoreBlocksPerSm) k_score(cons
     for(uint32_t c0 = 0; c0 < n_slots; c0 += kScoreThreads)
         {
             const uint32_t i = c0 + threadIdx.x;
-            uint32_t slices = 0;
-            if(i < n_slots && S[i].status == KGMT_QUERY_RUNNING && S[i].n_samples > 0 && P[i].regions > kScoreSmall)
-                slices = (P[i].regions + kScoreSlice - 1) / kScoreSlice;
+            const uint32_t slices = i < n_slots && has_large_table(P, S, i) ? (P[i].regions + kScoreSlice - 1) / kScoreSlice : 0u;
             uint32_t total;
             s_pre[threadIdx.x] = block_exclusive_scan<kScoreThreads>(slices, scratch, &total);
             if(threadIdx.x == 0) s_pre[kScoreThreads] = total;
@@ -554,21 +560,27 @@ __global__ void __launch_bounds__(kScoreThreads, kScoreBlocksPerSm) k_score(cons
             for(uint32_t j = (blockIdx.x + gridDim.x - before % gridDim.x) % gridDim.x; j < total; j += gridDim.x)
                 {
                     const int g = find_slot(s_pre, kScoreThreads, j);
-                    const uint32_t q = c0 + (uint32_t)g;
-                    const ScoreParams sp = score_params(P[q]);
-                    QueryState& st = S[q];
-                    score_slice<kScoreThreads>(sp, j - s_pre[g]);
-                    __syncthreads();
-                    if(threadIdx.x == 0) s_last = atomic_add_release(&st.score_done, 1u) == s_pre[g + 1] - s_pre[g] - 1u;
-                    __syncthreads();
-                    if(s_last)
-                        {
-                            __threadfence();
-                            if(threadIdx.x == 0) st.score_done = 0;
-                            score_finish<kScoreThreads>(sp, st, s_lanes);
-                        }
+                    score_slice<kScoreThreads>(score_params(P[c0 + (uint32_t)g]), j - s_pre[g]);
                 }
             before += total;
+            __syncthreads();
+        }
+    if(!waited) pdl_wait();
+}
+
+__global__ void __launch_bounds__(kSumThreads, kSumBlocksPerSm) k_score_sum(const QueryParams* __restrict__ P, QueryState* S, const Sched* sched)
+{
+    __shared__ float s_lanes[kScoreLanes];
+    pdl_trigger();
+    const uint32_t n_slots = sched->n_slots;
+    bool waited = false;
+    for(uint32_t q = blockIdx.x; q < n_slots; q += gridDim.x)
+        {
+            if(!has_large_table(P, S, q)) continue;
+            const ScoreParams sp = score_params(P[q]);
+            if(!waited) pdl_wait();
+            waited = true;
+            score_finish<kSumThreads>(sp, S[q], s_lanes);
             __syncthreads();
         }
     if(!waited) pdl_wait();
@@ -1173,8 +1185,11 @@ cudaError_t launch_append(const LaunchArgs& a, int grid, cudaStream_t s)
 cudaError_t launch_score(const LaunchArgs& a, int sms, cudaStream_t s)
 {
     cudaLaunchAttribute attr[1];
-    const cudaLaunchConfig_t cfg = dependent_config(sms * kScoreBlocksPerSm, kScoreThreads, 0, s, attr);
-    return cudaLaunchKernelEx(&cfg, k_score, a.params, a.states, (const Sched*)a.sched);
+    cudaLaunchConfig_t cfg = dependent_config(sms * kScoreBlocksPerSm, kScoreThreads, 0, s, attr);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_score, a.params, (const QueryState*)a.states, (const Sched*)a.sched);
+    if(e != cudaSuccess) return e;
+    cfg = dependent_config(sms * kSumBlocksPerSm, kSumThreads, 0, s, attr);
+    return cudaLaunchKernelEx(&cfg, k_score_sum, a.params, a.states, (const Sched*)a.sched);
 }
 
 cudaError_t launch_admit(const LaunchArgs& a, uint32_t first, uint32_t count, cudaStream_t s, const uint32_t* slots)

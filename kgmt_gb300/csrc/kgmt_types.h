@@ -16,13 +16,12 @@ namespace kgmt {
 constexpr int kMaxSampleDim = KGMT_MAX_SAMPLE_DIM;
 constexpr int kScoreLanes = 256;        // fixed summation shape of the score total
 // Region tables of more than kScoreSmall regions are scored by many blocks,
-// kScoreSlice regions each (k_score; phase 2 of the tail launch), smaller ones
-// by the block that finishes the query's last propagate tile.  One block took
-// 52 us an iteration for 32^3 regions and 6 for 16^3 (three divisions a region
-// on one SM), 1.5 for 8^3; in slices they take 10 and 4, of which about 2 are
-// the extra launch.
+// kScoreSlice regions each (k_score; the tail launch's scores), smaller ones by
+// the block that finishes the query's last propagate tile.  One block took 52 us
+// an iteration for 32^3 regions and 6 for 16^3 (three divisions a region on one
+// SM), 1.5 for 8^3.
 constexpr uint32_t kScoreSmall = 1024;
-constexpr uint32_t kScoreSlice = 2048;
+constexpr uint32_t kScoreSlice = 1024;
 constexpr int kTileC = 1024;            // samples per append tile
 constexpr int kAppendThreads = 256;     // threads per append block
 constexpr int kAppendPer = kTileC / kAppendThreads;  // samples per append thread
@@ -200,7 +199,7 @@ struct QueryState {
     uint32_t path_len;
     float goal_cost;      // the goal node's cost (set with the path)
     uint32_t path_at;     // first word of the path's rows in the host path buffer (kNoPath: not there)
-    uint32_t score_done;  // slices of a large region table scored this iteration
+    uint32_t pad;
     unsigned long long t_start;  // %globaltimer at admission (ns)
     unsigned long long t_end;
     unsigned long long steps;    // RK4 steps executed over all samples
