@@ -303,8 +303,8 @@ __device__ __forceinline__ int grid_cell(const QueryParams& P, float x)
 }
 
 // Where the culling grid of the current query lives: its starts (and the
-// first kSmemGridItems items) staged in shared memory by the propagate
-// kernel, the rest of the items in global memory.  start == nullptr: no grid.
+// first kSmemGridItems items) staged in shared memory by the kernel, the rest
+// of the items in global memory.  start == nullptr: no grid.
 struct GridView {
     const uint16_t* start;
     const uint16_t* items_s;

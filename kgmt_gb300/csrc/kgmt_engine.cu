@@ -475,7 +475,7 @@ kgmt_status Engine::set_prop_block(uint32_t block)
     KGMT_CUDA(cudaGetDevice(&dev), "cudaGetDevice");
     KGMT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
     sms_ = sms;
-    for(int m : {1, 2, 4, 8, 15}) grid_a_[m] = sms * propagate_blocks_per_sm((int)block, m);
+    prop_grid_for_ = 0;
     grid_c_ = sms * append_blocks_per_sm();
     // the tail launch: one block per SM (all blocks resident for its grid-wide
     // barriers), iterations up to two samples per thread
@@ -491,7 +491,7 @@ kgmt_status Engine::set_prop_block(uint32_t block)
     s.prop_block = block;
     // two samples per thread once an iteration fills the resident threads of
     // the double-integrator variant twice
-    s.pair_samples = 2u * (uint32_t)grid_a_[1] * block;
+    s.pair_samples = 2u * (uint32_t)(sms * propagate_blocks_per_sm((int)block, Engine::model_bit(KGMT_MODEL_DOUBLE_INTEGRATOR), kSmemBoxesMin)) * block;
     s.n_sms = (uint32_t)sms;
     s.old_tile = kTileOld;
     s.host_running = d_running_;
@@ -635,6 +635,19 @@ kgmt_status Engine::record_event(cudaEvent_t* out)
     return KGMT_OK;
 }
 
+// blocks of a propagate launch: all that are resident at once (queried when the
+// variant or the boxes it stages change)
+int Engine::propagate_grid()
+{
+    const uint32_t key = (uint32_t)models_ << 16 | smem_boxes_;
+    if(prop_grid_for_ != key)
+        {
+            prop_grid_ = sms_ * propagate_blocks_per_sm((int)prop_block_, models_, smem_boxes_);
+            prop_grid_for_ = key;
+        }
+    return prop_grid_;
+}
+
 kgmt_status Engine::launch_iteration()
 {
     const LaunchArgs a = args();
@@ -649,8 +662,8 @@ kgmt_status Engine::launch_iteration()
                 }
             if(k == 0)
                 {
-                    KGMT_CUDA(launch_propagate(a, (int)prop_block_, models_, grid_a_[models_], smem_boxes_, stream_), "k_propagate");
-                    if(large_tables_) KGMT_CUDA(launch_score(a, sms_, stream_), "k_score");
+                    KGMT_CUDA(launch_propagate(a, (int)prop_block_, models_, propagate_grid(), smem_boxes_, stream_), "k_propagate");
+                    KGMT_CUDA(launch_score(a, sms_, large_tables_, stream_), "k_score");
                 }
             else KGMT_CUDA(launch_append(a, grid_c_, stream_), "k_append");
             if(profile_)
@@ -659,7 +672,7 @@ kgmt_status Engine::launch_iteration()
                     if(st != KGMT_OK) return st;
                 }
         }
-    launches_ += large_tables_ ? 4 : 2;
+    launches_ += large_tables_ ? 4 : 3;
     return KGMT_OK;
 }
 
@@ -767,7 +780,7 @@ kgmt_status Engine::launch_unit()
                     if(st != KGMT_OK) return st;
                 }
             KGMT_CUDA(cudaGraphLaunch(graph_, stream_), "cudaGraphLaunch");
-            launches_ += (large_tables_ ? 4ull : 2ull) * iters_per_graph_;
+            launches_ += (large_tables_ ? 4ull : 3ull) * iters_per_graph_;
         }
     else
         {

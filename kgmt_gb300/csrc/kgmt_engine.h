@@ -156,6 +156,7 @@ class Engine {
 
    private:
     kgmt_status launch_iteration();
+    int propagate_grid();
     // one tail launch after what is queued, waited for; *done: nothing runs any more
     kgmt_status run_tail(bool* done, bool* declined_at_once);
     kgmt_status record_event(cudaEvent_t* out);
@@ -168,7 +169,8 @@ class Engine {
     uint32_t prop_block_ = 256;
     uint32_t iters_per_graph_ = 4;
     bool use_graph_ = true;
-    int grid_a_[16] = {};           // propagate grid per variant
+    int prop_grid_ = 0;             // blocks of a propagate launch
+    uint32_t prop_grid_for_ = 0;    // its variant and box capacity
     int grid_c_ = 0;
     int sms_ = 0;
     bool large_tables_ = true;      // the chain scores large region tables in their own launch

@@ -400,8 +400,7 @@ __device__ __forceinline__ void plan_samples(const QueryParams& P, QueryState& s
 }
 
 // ---------------------------------------------------------------------------
-// propagate (+ the region scores of each query, computed by the block that
-// finishes the query's last propagate tile)
+// propagate
 // ---------------------------------------------------------------------------
 struct PropCtx {
     uint32_t itr, spe, n_react, n_samples;
@@ -413,7 +412,6 @@ struct PropShared {
     uint32_t acc;                // accepted samples of the tile
     uint32_t steps;              // RK4 steps of the tile
     uint32_t tests;              // box tests of the tile
-    uint32_t next_run;           // runs of the sorted tile handed to warps so far
 };
 
 // sample rows of a model
@@ -594,112 +592,168 @@ __device__ __forceinline__ void finish_sample(const QueryParams& p, const GridVi
         }
 }
 
-// One propagate tile of `tile` samples of one query: tile <= NT (a power of
-// two) gives thread i < tile sample lt * tile + i; tile = kPropPer x NT gives
-// thread i samples (2 lt + h) * NT + i, h = 0, 1.  A counting sort of the tile
-// by step count (dead lanes last), then the sorted tile in runs of 32
-// consecutive samples, one sample a lane: a warp takes the longest run left
-// whenever it is free (a shared counter), so the warps of a block finish the
-// tile together however early their samples end.  `wait` runs once per
-// thread, after its first run has gathered its parents and draws (the boxes'
-// bulk copy may be in flight until then).  Block-uniform call.  COHERENT:
-// parent rows may have been appended by other blocks earlier in the same
-// launch (see load_row_ro).
-template <int NT, int MODELS, bool COHERENT = false, typename Wait>
-__device__ __forceinline__ void propagate_tile(const QueryParams& sp, const PropCtx& sc, uint32_t lt, uint32_t tile, uint32_t smem_boxes, PropShared* sh,
-                                               uint32_t* s_hist, uint32_t* s_perm, uint4* s_key, const float4* s_obs, const uint16_t* s_gstart,
-                                               const uint16_t* s_gitems, const uint32_t* s_gmeta, Wait&& wait)
+// ---------------------------------------------------------------------------
+// propagate tiles: each block keeps two, the one its warps work on and the next,
+// so a warp never waits for the block.  A tile's samples are counting-sorted by
+// step count and taken 32 at a time, longest first, by whichever warp is free;
+// the last warp to leave a tile adds up its counts and prepares the tile after
+// the next in the same buffer, while the others go on with the next.
+// Bound by instruction issue and, in small iterations, by the latency of the
+// few samples a warp has.  With block barriers around each tile the warps of a
+// block waited for its longest run and for the sort (2.6 - 2.9 of the 7 - 9
+// warps a scheduler had were at a barrier): iterations of the mixed batch with
+// few samples issued 40 - 48 % of the time, now 63 %; 256 double-integrator
+// queries took 3.12 ms, now 2.81; the 2M-node quadrotor tree 4.63, now 4.25.
+// ---------------------------------------------------------------------------
+template <int NT>
+struct TileBuf {
+    QueryParams p;  // of the tile's query
+    uint64_t bar;   // its boxes and grid, copied in bulk
+    PropCtx c;
+    int q;
+    uint32_t first, n;           // samples [first, first + n) of the query
+    uint32_t next_run, left;     // runs handed out; warps that are done with the tile
+    PropShared sh;
+    uint32_t hist[kSortBins];
+    uint16_t rank[kPropPer * NT];  // while sorting: step-count bin and rank in it
+    uint16_t perm[kPropPer * NT];  // samples in sorted order
+};
+
+// Tile `lt` of query q into a buffer, by one warp (BLOCK: by the whole block, for
+// a launch's first tile, which nothing overlaps): the query's params and loop
+// state, the bulk copies of its boxes and grid (not waited for), and the sorted
+// order.  dyn: the buffer's dynamic shared memory.
+template <int NT, int MODELS, bool BLOCK>
+__device__ __forceinline__ void prepare_tile(TileBuf<NT>& B, char* dyn, const QueryParams* __restrict__ P, const QueryState* S, int q, uint32_t lt,
+                                             uint32_t tile, uint32_t smem_boxes)
 {
-    const int model = sp.model;
-    const int per = tile > (uint32_t)NT ? kPropPer : 1;
-    {
-        uint32_t s0[kPropPer], rank[kPropPer];
-        int key[kPropPer];
-        U4 kb[kPropPer];
-        if(threadIdx.x < kSortBins) s_hist[threadIdx.x] = 0;
+    constexpr uint32_t W = BLOCK ? NT : 32;
+    const uint32_t lane = BLOCK ? threadIdx.x : threadIdx.x & 31u;
+    auto sync = [] {
+        if constexpr(BLOCK) __syncthreads();
+        else __syncwarp();
+    };
+    const unsigned full = 0xffffffffu;
+    const QueryParams& gp = P[q];
+    const uint32_t* src = (const uint32_t*)&gp;
+    uint32_t* dst = (uint32_t*)&B.p;
 #pragma unroll
-        for(int h = 0; h < kPropPer; ++h)
-            {
-                // with one sample per thread the second key is a dead lane
-                if(per == kPropPer) s0[h] = (lt * kPropPer + h) * NT + threadIdx.x;
-                else s0[h] = (h == 0 && threadIdx.x < tile) ? lt * tile + threadIdx.x : 0xFFFFFFFFu;
-                key[h] = kSortBins - 1;
-                kb[h] = U4{0u, 0u, 0u, 0u};
-                if(s0[h] < sc.n_samples)
-                    {
-                        int k = 1;
-                        with_model<MODELS>(model, [&](auto m) {
-                            kb[h] = sample_key_block<decltype(m)::value>(sp, sc, s0[h]);
-                            k = sample_steps<decltype(m)::value>(sp, kb[h]);
-                        });
-                        key[h] = k < kSortBins - 1 ? k : kSortBins - 2;
-                    }
-            }
-        __syncthreads();
+    for(uint32_t i = 0; i < (sizeof(QueryParams) / 4 + W - 1) / W; ++i)
+        if(i * W + lane < sizeof(QueryParams) / 4) dst[i * W + lane] = src[i * W + lane];
+    if(lane == 0)
+        {
+            const QueryState& st = S[q];
+            const uint32_t ns = st.n_samples;
+            B.c.itr = st.itr;
+            B.c.spe = st.spe;
+            B.c.n_react = st.n_react;
+            B.c.n_samples = ns;
+            B.q = q;
+            B.first = lt * tile;
+            B.n = min(tile, ns - lt * tile);
+            B.next_run = 0, B.left = 0;
+            B.sh.acc = 0, B.sh.steps = 0, B.sh.tests = 0;
+            // boxes, grid meta, grid starts and the first grid items: one
+            // mbarrier transaction of bulk copies (possibly of no bytes)
+            const uint32_t n_obs = gp.n_obstacles;
+            const bool obs_s = n_obs > 0 && n_obs <= smem_boxes;
+            const bool grid = gp.grid_meta != nullptr;
+            fence_proxy_async_smem();
+            mbar_expect_tx(&B.bar, (obs_s ? n_obs * 32u : 0u) + (grid ? 16u + kSmemStartBytes + kSmemGridItems * 2u : 0u));
+            if(obs_s) bulk_copy_g2s(dyn + kSmemGridBytes, gp.obstacles, n_obs * 32u, &B.bar);
+            if(grid)
+                {
+                    bulk_copy_g2s(dyn + kSmemStartBytes + kSmemGridItems * 2u, gp.grid_meta, 16u, &B.bar);
+                    bulk_copy_g2s(dyn, gp.grid_start, kSmemStartBytes, &B.bar);
+                    bulk_copy_g2s(dyn + kSmemStartBytes, gp.grid_items, kSmemGridItems * 2u, &B.bar);
+                }
+        }
+    if(lane < 32u) B.hist[lane] = 0;
+    static_assert(kSortBins == 32 && kPropPer * NT <= 1024, "a bin a lane; bin and rank share 16 bits");
+    sync();
+    const uint32_t n = B.n, first = B.first;
+    const int model = B.p.model;
+#pragma unroll 2
+    for(uint32_t i = lane; i < n; i += W)
+        {
+            int k = 1;
+            with_model<MODELS>(model, [&](auto m) {
+                constexpr int M = decltype(m)::value;
+                k = sample_steps<M>(B.p, sample_key_block<M>(B.p, B.c, first + i));
+            });
+            const uint32_t key = (uint32_t)(k < kSortBins ? k : kSortBins - 1);
+            B.rank[i] = (uint16_t)(key << 10 | atomicAdd(&B.hist[key], 1u));
+        }
+    sync();
+    if(!BLOCK || lane < 32u)
+        {
+    const uint32_t v = B.hist[lane];
+    uint32_t x = v;
 #pragma unroll
-        for(int h = 0; h < kPropPer; ++h) rank[h] = atomicAdd(&s_hist[key[h]], 1u);
-        __syncthreads();
-        if(threadIdx.x < 32)
-            {
-                // exclusive scan of the bins (kSortBins <= 32)
-                const uint32_t v = threadIdx.x < kSortBins ? s_hist[threadIdx.x] : 0u;
-                uint32_t x = v;
-#pragma unroll
-                for(int o = 1; o < 32; o <<= 1)
-                    {
-                        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-                        if(threadIdx.x >= (unsigned)o) x += y;
-                    }
-                if(threadIdx.x < kSortBins) s_hist[threadIdx.x] = x - v;
-            }
-        __syncthreads();
-#pragma unroll
-        for(int h = 0; h < kPropPer; ++h)
-            {
-                const uint32_t pos = s_hist[key[h]] + rank[h];
-                s_perm[pos] = s0[h];
-                s_key[pos] = make_uint4(kb[h].x, kb[h].y, kb[h].z, kb[h].w);
-            }
-        __syncthreads();
-    }
-    const float4* obs = sp.n_obstacles <= smem_boxes ? s_obs : sp.obstacles;
-    // live samples come first in the sorted order: the dead bin's start
-    const uint32_t n_live = s_hist[kSortBins - 1];
-    const uint32_t n_runs = (n_live + 31u) / 32u;
+    for(int o = 1; o < 32; o <<= 1)
+        {
+            const uint32_t y = __shfl_up_sync(full, x, o);
+            if(lane >= (uint32_t)o) x += y;
+        }
+    B.hist[lane] = x - v;
+        }
+    sync();
+    for(uint32_t i = lane; i < n; i += W)
+        {
+            const uint32_t r = B.rank[i];
+            B.perm[B.hist[r >> 10] + (r & 1023u)] = (uint16_t)i;
+        }
+}
+
+// The runs of a prepared tile that this warp takes.  parity: of the buffer's
+// bulk copies, waited for once, after the first run has gathered its parents.
+template <int NT, int MODELS>
+__device__ __forceinline__ void run_tile(TileBuf<NT>& B, char* dyn, uint32_t smem_boxes, uint32_t parity, uint32_t* error)
+{
     const unsigned full = 0xffffffffu;
     const uint32_t lane = threadIdx.x & 31u;
+    const QueryParams& sp = B.p;
+    const int model = sp.model;
+    const uint32_t n = B.n, n_runs = (n + 31u) / 32u;
+    const uint16_t* gstart = (const uint16_t*)dyn;
+    const uint16_t* gitems = (const uint16_t*)(dyn + kSmemStartBytes);
+    const uint32_t* gmeta = (const uint32_t*)(dyn + kSmemStartBytes + kSmemGridItems * 2u);
+    const float4* obs = sp.n_obstacles <= smem_boxes ? (const float4*)(dyn + kSmemGridBytes) : sp.obstacles;
     bool waited = false;
     for(;;)
         {
             uint32_t run = 0;
-            if(lane == 0) run = atomicAdd(&sh->next_run, 1u);
+            if(lane == 0) run = atomicAdd(&B.next_run, 1u);
             run = __shfl_sync(full, run, 0);
             if(run >= n_runs) break;
             // longest runs first
             const uint32_t slot = (n_runs - 1u - run) * 32u + lane;
-            const uint32_t s = slot < n_live ? s_perm[slot] : 0xFFFFFFFFu;
-            const bool live = s < sc.n_samples;
+            const bool live = slot < n;
+            const uint32_t s = B.first + (live ? (uint32_t)B.perm[slot] : 0u);
             float x0[KGMT_MAX_SAMPLE_DIM], u[8];
             uint32_t par = 0;
             if(live)
-                {
-                    const uint4 k4 = s_key[slot];
-                    const U4 kb1{k4.x, k4.y, k4.z, k4.w};
-                    with_model<MODELS>(model, [&](auto m) { par = prepare_sample<decltype(m)::value, COHERENT>(sp, sc, s, kb1, x0, u); });
-                }
+                with_model<MODELS>(model, [&](auto m) {
+                    constexpr int M = decltype(m)::value;
+                    par = prepare_sample<M>(sp, B.c, s, sample_key_block<M>(sp, B.c, s), x0, u);
+                });
             if(!waited)
                 {
-                    wait();
                     waited = true;
+                    uint32_t spins = 0;
+                    while(!mbar_try_wait(&B.bar, parity))
+                        if(++spins > kSpinLimit)
+                            {
+                                if(lane == 0) atomicOr(error, kErrCopyTimeout);
+                                break;
+                            }
                 }
-            const GridView grid{(sp.grid_meta != nullptr && s_gmeta[1] == 1u) ? s_gstart : nullptr, s_gitems, sp.grid_items};
+            const GridView grid{(sp.grid_meta != nullptr && gmeta[1] == 1u) ? gstart : nullptr, gitems, sp.grid_items};
             with_model<MODELS>(model, [&](auto m) {
                 constexpr int M = decltype(m)::value;
-                finish_sample<M>(sp, grid, obs, sp.n_obstacles, s, live, par, x0, u, sh, sp.us + (size_t)s * ModelDims<M>::D, sp.up + s, sp.ur1f + s);
+                finish_sample<M>(sp, grid, obs, sp.n_obstacles, s, live, par, x0, u, &B.sh, sp.us + (size_t)s * ModelDims<M>::D, sp.up + s, sp.ur1f + s);
             });
         }
-    // a thread that got no run still follows the copy's phase
-    if(!waited) wait();
 }
 
 // Samples [s0, s0 + n) of one query, one per thread (n <= NT), in index
@@ -970,7 +1024,6 @@ __device__ inline void finalize_query(const QueryParams& p, QueryState& st, Sche
     st.w_new = w_total;
     // per-iteration accumulators start from zero next iteration
     st.tiles_done = 0;
-    st.prop_done = 0;
     st.react_total = 0;
     st.acc_total = 0;
     st.w_total = 0;

@@ -1,17 +1,18 @@
 // kgmt_kernels.cu -- the per-iteration kernel chain of the KGMT planning loop.
 //
 // One iteration of every running query (reference: KGMT::plan loop body,
-// src/planners/KGMT.cu:84-95) is two launches with fixed shapes, so the
-// chain can be captured once in a CUDA graph and replayed:
+// src/planners/KGMT.cu:84-95) is three launches with fixed shapes (four where a
+// query has a large region table), so the chain can be captured once in a CUDA
+// graph and replayed:
 //
 //   k_propagate  KGMT::propagateFrontier + propagateFrontier_kernel1/2
 //                (KGMT.cu:167-299): one thread per sample, persistent blocks
 //                taking propagate tiles from a ticket counter, obstacles of
 //                the tile's query staged in shared memory by a bulk (TMA)
-//                copy, warp-aggregated atomics into the region histograms.
-//                The block that finishes a query's last propagate tile
-//                then runs Graph::updateVertices (Graph.cu:207-358) for that
-//                query: region scores summed in a fixed order.
+//                copy, one tile ahead; warp-aggregated counts.
+//   k_score      raw region scores of large tables, in slices.
+//   k_score_sum  Graph::updateVertices (Graph.cu:207-358): the other tables'
+//                scores; sums in a fixed order, normalisation.
 //   k_append     KGMT::updateFrontier + updateFrontier_kernel
 //                (KGMT.cu:305-403) and the next iteration's frontier
 //                compaction / repeat expansion (KGMT.cu:167-181,
@@ -21,6 +22,10 @@
 //                re-activated node its frontier slot; the last tile of a
 //                query finalises it, the last query computes the schedule of
 //                the next iteration on the device.
+//
+// Before the first iteration k_begin (one query) or k_admit and k_build_grid lay
+// out a query; k_tail (kgmt_tail.cuh) runs the iterations of few and small
+// queries in one launch; k_paths reads the found paths out.
 //
 // Frontier representation: instead of frontier flags over the whole tree and
 // two scans per iteration (KGMT.cu:170-181), the frontier of the next
@@ -386,24 +391,14 @@ template <int NT, int MODELS>
 __global__ void __launch_bounds__(NT, (MODELS == kBitDI ? 1024 : 512) / NT) k_propagate(const QueryParams* __restrict__ P, QueryState* S, Sched* sched,
                                                   const uint32_t* __restrict__ tile_base, uint32_t smem_boxes)
 {
-    // dynamic shared memory: grid starts | grid items | grid meta | boxes
-    // (smem_boxes of them; a query with more reads its boxes from global memory)
+    // dynamic shared memory of each of the two buffers: grid starts | grid
+    // items | grid meta | boxes (smem_boxes of them; a query with more reads
+    // its boxes from global memory)
     extern __shared__ float4 s_dyn[];
-    uint16_t* s_gstart = (uint16_t*)s_dyn;
-    uint16_t* s_gitems = (uint16_t*)((char*)s_dyn + kSmemStartBytes);
-    uint32_t* s_gmeta = (uint32_t*)((char*)s_dyn + kSmemStartBytes + kSmemItemBytes);
-    float4* s_obs = (float4*)((char*)s_dyn + kSmemGridBytes);
-    __shared__ uint32_t s_copy;
-    __shared__ alignas(8) uint64_t bar;
-    __shared__ QueryParams s_p;
-    __shared__ PropCtx s_c;
-    __shared__ PropShared s_sh;
-    __shared__ float s_lanes[kScoreLanes];
+    __shared__ TileBuf<NT> s_buf[2];
+    __shared__ volatile uint32_t s_ready[2];  // 1 + the number of the block's tile in the buffer, or kEnd
     __shared__ uint32_t s_base[kBaseCache];
-    __shared__ uint32_t s_hist[kSortBins];
-    __shared__ uint32_t s_perm[kPropPer * NT];
-    __shared__ uint4 s_key[kPropPer * NT];  // key Philox block of each sorted sample
-    __shared__ int s_tile, s_q, s_last;
+    constexpr uint32_t kEnd = 0xFFFFFFFFu, NW = NT / 32;
     // everything here depends on the append kernel before this one (its
     // schedule, frontier and tree); once that is complete the append kernel
     // after this one may be scheduled into the SMs this launch leaves free
@@ -422,108 +417,94 @@ __global__ void __launch_bounds__(NT, (MODELS == kBitDI ? 1024 : 512) / NT) k_pr
     if(blockIdx.x >= total) return;
     if(threadIdx.x == 0)
         {
-            mbar_init(&bar, 1);
+            mbar_init(&s_buf[0].bar, 1);
+            mbar_init(&s_buf[1].bar, 1);
+            s_ready[0] = 0, s_ready[1] = 0;
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
     const BaseCache bases = cache_bases(tile_base, n_slots, s_base);
-    int cur_q = -1;
-    uint32_t phase = 0;
-    uint32_t t = blockIdx.x;  // first tile static, then tickets
-    uint32_t t_next = 0;      // ticket taken while the current tile runs (thread 0)
-    for(;;)
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    auto dyn = [&](uint32_t i) { return (char*)s_dyn + (i & 1u) * (prop_smem_bytes(smem_boxes) / 2); };
+    // the block's tile number i, tile t of the iteration; by one warp
+    auto prepare = [&](uint32_t i, uint32_t t) {
+        if(t < total)
+            {
+                const int q = find_slot(bases.base, bases.n, t);
+                prepare_tile<NT, MODELS, false>(s_buf[i & 1u], dyn(i), P, S, q, t - bases.base[q], tile, smem_boxes);
+            }
+        __syncwarp();
+        if(lane == 0)
+            {
+                __threadfence_block();
+                s_ready[i & 1u] = t < total ? i + 1u : kEnd;
+            }
+    };
+    // first tile static, then tickets
+    auto ticket = [&] {
+        uint32_t t = 0;
+        if(lane == 0) t = gridDim.x + atomicAdd(&sched->ticket_a, 1u);
+        return __shfl_sync(0xffffffffu, t, 0);
+    };
+    {
+        const int q = find_slot(bases.base, bases.n, blockIdx.x);
+        prepare_tile<NT, MODELS, true>(s_buf[0], dyn(0), P, S, q, blockIdx.x - bases.base[q], tile, smem_boxes);
+    }
+    if(threadIdx.x == 0) s_ready[0] = 1u;
+    __syncthreads();
+    if(warp == 0) prepare(1, ticket());
+    for(uint32_t i = 0;; ++i)
         {
-            if(threadIdx.x == 0)
+            TileBuf<NT>& B = s_buf[i & 1u];
+            uint32_t r = 0;
+            if(lane == 0)
                 {
-                    s_tile = (int)t;
-                    s_q = t < total ? find_slot(bases.base, bases.n, t) : -1;
-                    s_sh.acc = 0, s_sh.steps = 0, s_sh.tests = 0, s_sh.next_run = 0;
-                    s_last = 0;
-                    if(t < total) t_next = gridDim.x + atomicAdd(&sched->ticket_a, 1u);
-                }
-            __syncthreads();
-            t = (uint32_t)s_tile;
-            if(t >= total) break;
-            const int q = s_q;
-            bool wait_obs = false;
-            if(q != cur_q)
-                {
-                    // stage the query's parameters; its boxes go by bulk copy
-                    const uint32_t* src = (const uint32_t*)&P[q];
-                    uint32_t* dst = (uint32_t*)&s_p;
-                    for(int i = threadIdx.x; i < (int)(sizeof(QueryParams) / 4); i += NT) dst[i] = src[i];
-                    if(threadIdx.x == 0)
+                    uint32_t spins = 0;
+                    while((r = s_ready[i & 1u]) != i + 1u && r != kEnd)
                         {
-                            const QueryState& st = S[q];
-                            s_c.itr = st.itr;
-                            s_c.spe = st.spe;
-                            s_c.n_react = st.n_react;
-                            s_c.n_samples = st.n_samples;
-                            // boxes, grid meta, grid starts and the first grid
-                            // items: one mbarrier transaction of bulk copies
-                            const QueryParams& gp = P[q];
-                            const uint32_t n_obs = gp.n_obstacles;
-                            const bool obs_s = n_obs > 0 && n_obs <= smem_boxes;
-                            const bool grid = gp.grid_meta != nullptr;
-                            const uint32_t bytes = (obs_s ? n_obs * 32u : 0u) + (grid ? 16u + kSmemStartBytes + kSmemItemBytes : 0u);
-                            s_copy = bytes;
-                            if(bytes)
+                            if(++spins > kSpinLimit)
                                 {
-                                    fence_proxy_async_smem();
-                                    mbar_expect_tx(&bar, bytes);
-                                    if(obs_s) bulk_copy_g2s(s_obs, gp.obstacles, n_obs * 32u, &bar);
-                                    if(grid)
-                                        {
-                                            bulk_copy_g2s(s_gmeta, gp.grid_meta, 16u, &bar);
-                                            bulk_copy_g2s(s_gstart, gp.grid_start, kSmemStartBytes, &bar);
-                                            bulk_copy_g2s(s_gitems, gp.grid_items, kSmemItemBytes, &bar);
-                                        }
+                                    atomicOr(&sched->error, kErrCopyTimeout);
+                                    r = kEnd;
+                                    break;
                                 }
+                            __nanosleep(20);
                         }
-                    __syncthreads();
-                    wait_obs = s_copy != 0;
-                    cur_q = q;
+                    __threadfence_block();
                 }
-            const uint32_t lt = t - bases.base[q];
-            propagate_tile<NT, MODELS>(s_p, s_c, lt, tile, smem_boxes, &s_sh, s_hist, s_perm, s_key, s_obs, s_gstart, s_gitems, s_gmeta, [&] {
-                if(!wait_obs) return;
-                uint32_t spins = 0;
-                while(!mbar_try_wait(&bar, phase))
-                    if(++spins > kSpinLimit)
+            if(__shfl_sync(0xffffffffu, r, 0) == kEnd) break;
+            __syncwarp();
+            run_tile<NT, MODELS>(B, dyn(i), smem_boxes, (i >> 1) & 1u, &sched->error);
+            // the last warp to leave has the whole tile behind it
+            __syncwarp();
+            uint32_t last = 0;
+            if(lane == 0)
+                {
+                    __threadfence_block();
+                    last = atomicAdd(&B.left, 1u) == NW - 1u;
+                    if(last)
                         {
-                            if(threadIdx.x == 0) atomicOr(&sched->error, kErrCopyTimeout);
-                            break;
+                            __threadfence_block();
+                            QueryState& st = S[B.q];
+                            if(B.sh.acc) atomicAdd(&st.n_next, B.sh.acc);
+                            if(B.sh.steps) atomicAdd(&st.steps, (unsigned long long)B.sh.steps);
+                            if(B.sh.tests) atomicAdd(&st.tests, (unsigned long long)B.sh.tests);
                         }
-                phase ^= 1u;
-            });
-            __syncthreads();
-            if(threadIdx.x == 0)
-                {
-                    QueryState& st = S[q];
-                    if(s_sh.acc) atomicAdd(&st.n_next, s_sh.acc);
-                    if(s_sh.steps) atomicAdd(&st.steps, (unsigned long long)s_sh.steps);
-                    if(s_sh.tests) atomicAdd(&st.tests, (unsigned long long)s_sh.tests);
-                    const uint32_t n_tiles = bases.base[q + 1] - bases.base[q];
-                    if(atomic_add_release(&st.prop_done, 1u) == n_tiles - 1) s_last = 1;
-                    t = t_next;
-                    s_tile = (int)t;
                 }
-            __syncthreads();
-            if(s_last && s_p.regions <= kScoreSmall)
-                {
-                    __threadfence();
-                    update_scores<NT>(score_params(s_p), S[q], s_lanes);
-                }
-            t = (uint32_t)s_tile;
-            __syncthreads();
+            last = __shfl_sync(0xffffffffu, last, 0);
+            __syncwarp();
+            if(last) prepare(i + 2u, ticket());
         }
 }
 
-// Region scores of the queries with large tables, between the propagate and the
-// append launch (only in chains that hold such a query): k_score, raw scores,
-// the slices of all queries round the blocks; k_score_sum, total and
-// normalisation, one block a query.  Bound by L2 and DRAM latency.  As one launch
-// in which the block that finished a query's last slice summed it, 190 queries of
-// up to 32^3 regions took 75 us (some blocks summed three of them), now 27 + 16.
+// Region scores, between the propagate and the append launch.  k_score (only in
+// chains with a query of more than kScoreSmall regions): raw scores of the large
+// tables, their slices round the blocks.  k_score_sum: one block a query scores a
+// small table whole, or sums and normalises a large one.  Bound by L2 and DRAM
+// latency.  As one launch in which the block that finished a query's last slice
+// summed it, 190 queries of up to 32^3 regions took 75 us (some blocks summed
+// three of them), now 27 + 19.  (Small tables scored by the propagate block that
+// finished the query held that block's next tile up.)
 constexpr int kScoreThreads = 256;
 constexpr int kScoreBlocksPerSm = 6;
 constexpr int kSumThreads = 512;
@@ -576,11 +557,12 @@ __global__ void __launch_bounds__(kSumThreads, kSumBlocksPerSm) k_score_sum(cons
     bool waited = false;
     for(uint32_t q = blockIdx.x; q < n_slots; q += gridDim.x)
         {
-            if(!has_large_table(P, S, q)) continue;
+            if(S[q].status != KGMT_QUERY_RUNNING || S[q].n_samples == 0) continue;
             const ScoreParams sp = score_params(P[q]);
             if(!waited) pdl_wait();
             waited = true;
-            score_finish<kSumThreads>(sp, S[q], s_lanes);
+            if(sp.regions > kScoreSmall) score_finish<kSumThreads>(sp, S[q], s_lanes);
+            else update_scores<kSumThreads>(sp, S[q], s_lanes);
             __syncthreads();
         }
     if(!waited) pdl_wait();
@@ -1130,11 +1112,11 @@ cudaError_t launch_propagate(const LaunchArgs& a, int block, int models, int gri
 // shared memory on top of more than 48 KB in total (the launch wrappers run
 // after this has been called for the variant)
 template <int NT, int MODELS>
-static int occupancy_t()
+static int occupancy_t(uint32_t boxes)
 {
     int n = 0;
-    const size_t smem = kPropSmemBytes;
-    if(cudaFuncSetAttribute(k_propagate<NT, MODELS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    const size_t smem = prop_smem_bytes(boxes);
+    if(cudaFuncSetAttribute(k_propagate<NT, MODELS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prop_smem_bytes(kSmemObstacles)) != cudaSuccess)
         {
             cudaGetLastError();
             return 0;
@@ -1144,26 +1126,26 @@ static int occupancy_t()
 }
 
 template <int NT>
-static int occupancy_m(int models)
+static int occupancy_m(int models, uint32_t boxes)
 {
     switch(models)
         {
-            case kBitDI: return occupancy_t<NT, kBitDI>();
-            case kBitQuad: return occupancy_t<NT, kBitQuad>();
-            case kBitDubins: return occupancy_t<NT, kBitDubins>();
-            case kBitUnicycle: return occupancy_t<NT, kBitUnicycle>();
-            default: return occupancy_t<NT, kAllModels>();
+            case kBitDI: return occupancy_t<NT, kBitDI>(boxes);
+            case kBitQuad: return occupancy_t<NT, kBitQuad>(boxes);
+            case kBitDubins: return occupancy_t<NT, kBitDubins>(boxes);
+            case kBitUnicycle: return occupancy_t<NT, kBitUnicycle>(boxes);
+            default: return occupancy_t<NT, kAllModels>(boxes);
         }
 }
 
-int propagate_blocks_per_sm(int block, int models)
+int propagate_blocks_per_sm(int block, int models, uint32_t boxes)
 {
     int n = 0;
     switch(block)
         {
-            case 128: n = occupancy_m<128>(models); break;
-            case 512: n = occupancy_m<512>(models); break;
-            default: n = occupancy_m<256>(models); break;
+            case 128: n = occupancy_m<128>(models, boxes); break;
+            case 512: n = occupancy_m<512>(models, boxes); break;
+            default: n = occupancy_m<256>(models, boxes); break;
         }
     return n > 0 ? n : 1;
 }
@@ -1182,12 +1164,16 @@ cudaError_t launch_append(const LaunchArgs& a, int grid, cudaStream_t s)
     return cudaLaunchKernelEx(&cfg, k_append, a.params, a.states, a.sched, a.tile_a_base, a.tile_c_base, a.tile_c_old);
 }
 
-cudaError_t launch_score(const LaunchArgs& a, int sms, cudaStream_t s)
+cudaError_t launch_score(const LaunchArgs& a, int sms, bool large, cudaStream_t s)
 {
     cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg = dependent_config(sms * kScoreBlocksPerSm, kScoreThreads, 0, s, attr);
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_score, a.params, (const QueryState*)a.states, (const Sched*)a.sched);
-    if(e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg;
+    if(large)
+        {
+            cfg = dependent_config(sms * kScoreBlocksPerSm, kScoreThreads, 0, s, attr);
+            const cudaError_t e = cudaLaunchKernelEx(&cfg, k_score, a.params, (const QueryState*)a.states, (const Sched*)a.sched);
+            if(e != cudaSuccess) return e;
+        }
     cfg = dependent_config(sms * kSumBlocksPerSm, kSumThreads, 0, s, attr);
     return cudaLaunchKernelEx(&cfg, k_score_sum, a.params, a.states, (const Sched*)a.sched);
 }

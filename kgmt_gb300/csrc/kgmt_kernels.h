@@ -22,9 +22,9 @@ cudaError_t launch_schedule(const LaunchArgs& a, cudaStream_t s);
 // smem_boxes: boxes a block stages in shared memory (the largest query of the
 // launch, rounded by smem_boxes_for); more are read from global memory
 cudaError_t launch_propagate(const LaunchArgs& a, int block, int models, int grid, uint32_t smem_boxes, cudaStream_t s);
-// region scores of queries with more than kScoreSmall regions (between propagate
-// and append; needed when the launch may meet such a query)
-cudaError_t launch_score(const LaunchArgs& a, int sms, cudaStream_t s);
+// region scores, between propagate and append; large: whether some query has
+// more than kScoreSmall regions
+cudaError_t launch_score(const LaunchArgs& a, int sms, bool large, cudaStream_t s);
 cudaError_t launch_append(const LaunchArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_paths(const LaunchArgs& a, uint32_t n, const HostSink& sink, cudaStream_t s);
 // admission of the engine's only query in one launch: its params (by value,
@@ -40,7 +40,8 @@ uint32_t bounds_error_take();
 cudaError_t launch_selftest_wait(unsigned long long* tiles, uint32_t* error, uint32_t polls, cudaStream_t s);
 cudaError_t launch_propagate_samples(const QueryParams& p, const float* x0, const float* u, const float* obs, uint32_t n_obs, uint32_t n,
                                      float* x1, uint8_t* valid, int32_t* r1, int32_t* r2, cudaStream_t s);
-int propagate_blocks_per_sm(int block, int models);
+// boxes: that a launch stages
+int propagate_blocks_per_sm(int block, int models, uint32_t boxes);
 int append_blocks_per_sm();
 
 // persistent tail launch (kgmt_tail.cuh): whole iterations for at most

@@ -2,7 +2,7 @@
 // batches with few running queries and single plans.
 //
 // While at most kTailQueries queries run and an iteration is a few samples a
-// resident thread, the two-kernel chain's time is latency: launches, the
+// resident thread, the time of the chain of launches is latency: launches, the
 // schedule round trip, the look-back hand-overs of the ordered append.  k_tail
 // runs those iterations back to back inside one cooperative launch of one block
 // per SM.  Each iteration the running queries split the blocks twice, in
@@ -239,7 +239,7 @@ constexpr uint32_t kTailBitWords = 16;  // words of re-activation bits a thread 
 // at most `dim` floats
 __host__ __device__ constexpr uint32_t tail_smem_bytes(uint32_t boxes, uint32_t dim)
 {
-    return prop_smem_bytes(boxes) + kTailShare * dim * 4u + kTailBitWords * (uint32_t)kTailThreads * 4u;
+    return staged_bytes(boxes) + kTailShare * dim * 4u + kTailBitWords * (uint32_t)kTailThreads * 4u;
 }
 
 template <int MODELS>
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
     extern __shared__ float4 s_dyn[];
     uint16_t* s_gstart = (uint16_t*)s_dyn;
     uint16_t* s_gitems = (uint16_t*)((char*)s_dyn + kSmemStartBytes);
-    uint32_t* s_gmeta = (uint32_t*)((char*)s_dyn + kSmemStartBytes + kSmemItemBytes);
+    uint32_t* s_gmeta = (uint32_t*)((char*)s_dyn + kSmemStartBytes + kSmemGridItems * 2);
     float4* s_obs = (float4*)((char*)s_dyn + kSmemGridBytes);
     __shared__ uint32_t s_copy;
     __shared__ alignas(8) uint64_t mbar;
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
     __shared__ int s_score_q, s_qs, s_qn, s_nr, s_too_large;
     // the block's samples of this iteration: accepted end rows (dynamic, behind
     // the boxes), parents, and region words with the accept flag
-    float* s_rows = (float*)((char*)s_dyn + prop_smem_bytes(smem_boxes));
+    float* s_rows = (float*)((char*)s_dyn + staged_bytes(smem_boxes));
     uint32_t* s_bits = (uint32_t*)(s_rows + kTailShare * tail_row_dim<MODELS>());
     __shared__ int32_t s_par[kTailShare];
     __shared__ uint32_t s_word[kTailShare];
@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                                     s_too_large = tot > max_samples || big;
                                     s_qs = here;
                                     s_score_q = mine ? __ffs((int)mine) - 1 : -1;
-                                    s_sh.acc = 0, s_sh.steps = 0, s_sh.tests = 0, s_sh.next_run = 0;
+                                    s_sh.acc = 0, s_sh.steps = 0, s_sh.tests = 0;
                                     s_goal_min = kNone;
                                 }
                             else s_qn = here;
@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                                     const uint32_t n_obs = gp.n_obstacles;
                                     const bool obs_s = n_obs > 0 && n_obs <= smem_boxes;
                                     const bool grid = gp.grid_meta != nullptr;
-                                    const uint32_t bytes = (obs_s ? n_obs * 32u : 0u) + (grid ? 16u + kSmemStartBytes + kSmemItemBytes : 0u);
+                                    const uint32_t bytes = (obs_s ? n_obs * 32u : 0u) + (grid ? 16u + kSmemStartBytes + kSmemGridItems * 2 : 0u);
                                     s_copy = bytes;
                                     if(bytes)
                                         {
@@ -486,7 +486,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                                                 {
                                                     bulk_copy_g2s(s_gmeta, gp.grid_meta, 16u, &mbar);
                                                     bulk_copy_g2s(s_gstart, gp.grid_start, kSmemStartBytes, &mbar);
-                                                    bulk_copy_g2s(s_gitems, gp.grid_items, kSmemItemBytes, &mbar);
+                                                    bulk_copy_g2s(s_gitems, gp.grid_items, kSmemGridItems * 2, &mbar);
                                                 }
                                         }
                                 }

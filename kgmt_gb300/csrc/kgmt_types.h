@@ -88,17 +88,20 @@ constexpr uint32_t kGridCells = kGridDim * kGridDim * kGridDim;
 constexpr uint32_t kGridMaxVisit = 8;       // cells a step box may visit before falling back to all boxes
 constexpr uint32_t kMaxObstacles = 65535;   // grid items are 16-bit box indices
 constexpr uint32_t kMaxGridItems = 65535;   // grid starts are 16-bit
-constexpr uint32_t kSmemGridItems = 4096;   // grid items staged in shared memory per block
-// dynamic shared memory of k_propagate: grid starts, grid items, grid meta,
+// dynamic shared memory of a staged query: grid starts, grid items, grid meta,
 // then the boxes -- as many as the launch's box capacity, a power of two
 // from kSmemBoxesMin to kSmemObstacles sized to the admitted queries (what
-// shared memory the boxes leave unused stays L1 cache)
+// shared memory the boxes leave unused stays L1 cache).  k_propagate has it
+// twice, four blocks an SM.  Propagate launches of 64 double-integrator queries,
+// with 2048 / 3072 / 3584 / 4096 items: of 50 boxes 0.98 / 0.98 / 0.98 / 1.09 ms
+// (too little L1 is left), of 200 boxes 1.19 / 1.14 / 1.14 / 1.13, of 3000 2.26 /
+// 2.23 / 2.09 / 2.08.
+constexpr uint32_t kSmemGridItems = 3584;
 constexpr uint32_t kSmemStartBytes = ((kGridCells + 1) * 2 + 15) / 16 * 16;
-constexpr uint32_t kSmemItemBytes = kSmemGridItems * 2;
-constexpr uint32_t kSmemGridBytes = kSmemStartBytes + kSmemItemBytes + 16;
 constexpr uint32_t kSmemBoxesMin = 64;
-constexpr uint32_t kPropSmemBytes = kSmemGridBytes + kSmemObstacles * 32;  // the largest launch
-__host__ __device__ constexpr uint32_t prop_smem_bytes(uint32_t boxes) { return kSmemGridBytes + boxes * 32; }
+constexpr uint32_t kSmemGridBytes = kSmemStartBytes + kSmemGridItems * 2 + 16;
+__host__ __device__ constexpr uint32_t staged_bytes(uint32_t boxes) { return kSmemGridBytes + boxes * 32; }
+__host__ __device__ constexpr uint32_t prop_smem_bytes(uint32_t boxes) { return 2 * staged_bytes(boxes); }
 // box capacity for queries of at most max_obs boxes
 inline uint32_t smem_boxes_for(uint32_t max_obs)
 {
@@ -189,7 +192,6 @@ struct QueryState {
     int32_t goal_cand;    // smallest new tree index in the goal ball (atomicMin)
     int32_t goal_index;
     uint32_t tiles_done;  // append/re-activation tiles finished this iteration
-    uint32_t prop_done;   // propagate tiles finished this iteration
     uint32_t react_total; // atomics of the append kernel
     uint32_t acc_total;
     uint32_t w_total;
@@ -199,7 +201,6 @@ struct QueryState {
     uint32_t path_len;
     float goal_cost;      // the goal node's cost (set with the path)
     uint32_t path_at;     // first word of the path's rows in the host path buffer (kNoPath: not there)
-    uint32_t pad;
     unsigned long long t_start;  // %globaltimer at admission (ns)
     unsigned long long t_end;
     unsigned long long steps;    // RK4 steps executed over all samples
