@@ -87,7 +87,8 @@ class Engine {
     // the pieces of admit, for callers that admit several slot ranges
     kgmt_status upload_params(uint32_t first, uint32_t count);
     kgmt_status init_slots(uint32_t first, uint32_t count, const float* d_inits = nullptr, const float* d_goals = nullptr);
-    kgmt_status set_active(uint32_t n_active);
+    // order: the slots in the order their propagate tiles are taken (device memory; null: slot order)
+    kgmt_status set_active(uint32_t n_active, const uint32_t* order = nullptr);
     kgmt_status schedule();
     // runs iterations until no query is running (or max_iters + slack)
     kgmt_status run_until_done(uint32_t max_iters);
@@ -180,6 +181,8 @@ class Engine {
     QueryState* d_states_ = nullptr;
     Sched* d_sched_ = nullptr;
     uint32_t* d_tile_a_ = nullptr;
+    uint32_t* d_order_ = nullptr;
+    std::vector<uint32_t> h_order_;
     uint32_t* d_tile_c_ = nullptr;
     uint32_t* d_tile_old_ = nullptr;
     uint32_t* d_slot_list_ = nullptr;  // [slots] slots of a served admission

@@ -226,6 +226,7 @@ __device__ void compute_schedule(const QueryParams* __restrict__ P, const QueryS
     const uint32_t block = sched->prop_block;
     const uint32_t pair_samples = sched->pair_samples;
     const uint32_t sms = sched->n_sms;
+    const uint32_t* order = sched->prop_order;  // tile_a_base is in this order
     // samples per propagate tile: pairs per thread for large iterations; for
     // small ones the smallest power of two from 32 up to the block that keeps
     // the tiles within one per SM, so each tile's warps have an SM to
@@ -291,11 +292,12 @@ __device__ void compute_schedule(const QueryParams* __restrict__ P, const QueryS
                     const uint32_t tot_s = __reduce_add_sync(full, ns < kClamp ? ns : kClamp);
                     const uint32_t tot_t = __reduce_add_sync(full, tree < kClamp ? tree : kClamp);
                     const uint32_t prop_tile = tile_for(tot_s), old_tile = old_tile_for(tot_t);
-                    uint32_t ta = 0, tc = 0, told = 0;
+                    uint32_t tc = 0, told = 0;
+                    const uint32_t ns_a = __shfl_sync(full, ns, order && q < n ? (int)order[q] : q);
+                    // tile sizes are powers of two
+                    const uint32_t ta = (ns_a + prop_tile - 1) >> (__ffs(prop_tile) - 1);
                     if(run)
                         {
-                            // tile sizes are powers of two
-                            ta = (ns + prop_tile - 1) >> (__ffs(prop_tile) - 1);
                             told = (tree + old_tile - 1) >> (__ffs(old_tile) - 1);
                             tc = told + (ns + kTileC - 1) / kTileC;
                         }
@@ -352,10 +354,11 @@ __device__ void compute_schedule(const QueryParams* __restrict__ P, const QueryS
             const int q = base + (int)threadIdx.x;
             uint32_t ns = ns0, tree = tree0, run = run0;
             if(base > 0) run = load(q, ns, tree);
-            uint32_t ta = 0, tc = 0, told = 0;
+            uint32_t ns_a = ns, tree_a, tc = 0, told = 0;
+            if(order && q < n) load((int)order[q], ns_a, tree_a);
+            const uint32_t ta = (ns_a + prop_tile - 1) >> sh_a;
             if(run)
                 {
-                    ta = (ns + prop_tile - 1) >> sh_a;
                     told = (tree + old_tile - 1) >> sh_o;
                     tc = told + (ns + kTileC - 1) / kTileC;
                 }

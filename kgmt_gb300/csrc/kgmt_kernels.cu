@@ -414,6 +414,7 @@ __global__ void __launch_bounds__(NT, (MODELS == kBitDI ? 1024 : 512) / NT) k_pr
     const int n_slots = (int)sched->n_slots;
     // samples per tile this iteration (the schedule sized the tiles)
     const uint32_t tile = sched->prop_tile;
+    const uint32_t* order = sched->prop_order;
     if(blockIdx.x >= total) return;
     if(threadIdx.x == 0)
         {
@@ -430,8 +431,8 @@ __global__ void __launch_bounds__(NT, (MODELS == kBitDI ? 1024 : 512) / NT) k_pr
     auto prepare = [&](uint32_t i, uint32_t t) {
         if(t < total)
             {
-                const int q = find_slot(bases.base, bases.n, t);
-                prepare_tile<NT, MODELS, false>(s_buf[i & 1u], dyn(i), P, S, q, t - bases.base[q], tile, smem_boxes);
+                const int at = find_slot(bases.base, bases.n, t);
+                prepare_tile<NT, MODELS, false>(s_buf[i & 1u], dyn(i), P, S, order ? (int)order[at] : at, t - bases.base[at], tile, smem_boxes);
             }
         __syncwarp();
         if(lane == 0)
@@ -447,8 +448,8 @@ __global__ void __launch_bounds__(NT, (MODELS == kBitDI ? 1024 : 512) / NT) k_pr
         return __shfl_sync(0xffffffffu, t, 0);
     };
     {
-        const int q = find_slot(bases.base, bases.n, blockIdx.x);
-        prepare_tile<NT, MODELS, true>(s_buf[0], dyn(0), P, S, q, blockIdx.x - bases.base[q], tile, smem_boxes);
+        const int at = find_slot(bases.base, bases.n, blockIdx.x);
+        prepare_tile<NT, MODELS, true>(s_buf[0], dyn(0), P, S, order ? (int)order[at] : at, blockIdx.x - bases.base[at], tile, smem_boxes);
     }
     if(threadIdx.x == 0) s_ready[0] = 1u;
     __syncthreads();

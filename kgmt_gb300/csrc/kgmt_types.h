@@ -232,6 +232,8 @@ struct Sched {
     // the stream between graph replays: [0] mirrors `running`, [4] the samples
     // of the next iteration (clamped to 2^22)
     uint32_t* host_running;
+    // slots in the order their propagate tiles are taken (null: slot order)
+    const uint32_t* prop_order;
 };
 
 constexpr uint32_t kNoPath = 0xFFFFFFFFu;

@@ -52,3 +52,13 @@ def test_all_models(block, monkeypatch):
     for i, q in enumerate(qs):
         q.config = q.config.replace(max_iterations=8 + 2 * i)
     check(qs, monkeypatch, block)
+
+
+@pytest.mark.parametrize("n", [2, 32, 33, 256, 257, 300])
+def test_order_of_models(n, monkeypatch):
+    """Tiles are taken model by model: slots around a warp's and a block's number
+    of them, queries ending at different iterations."""
+    qs = W.all_models_batch(n, seed=n, tree_capacity=500)
+    for i, q in enumerate(qs):
+        q.config = q.config.replace(tree_capacity=300 + 40 * (i % 9), max_iterations=3 + i % 4, coarse_len=4, fine_len=2)
+    check(qs, monkeypatch)
