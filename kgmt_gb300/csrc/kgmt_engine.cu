@@ -673,7 +673,7 @@ int Engine::propagate_grid()
 kgmt_status Engine::launch_iteration()
 {
     const LaunchArgs a = args();
-    // kernel kinds in the profile: 0 propagate (with the region scores and k_score), 2 append
+    // kernel kinds in the profile: 0 propagate (with the score launches), 2 append
     for(int k = 0; k < 3; k += 2)
         {
             if(profile_)

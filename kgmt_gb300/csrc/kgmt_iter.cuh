@@ -790,10 +790,10 @@ __device__ __forceinline__ void propagate_range(const QueryParams& sp, const Pro
     });
 }
 
-// Graph::updateVertices (Graph.cu:311-358) for one query, by one block: all
-// regions scored, lane l of kScoreLanes sums regions l, l+256, ... in order,
-// then a halving tree over the lanes.  Histograms and marks were updated by
-// other blocks' atomics in this kernel: read past L1.
+// Graph::updateVertices (Graph.cu:311-358) for one query: all regions scored,
+// lane l of kScoreLanes sums regions l, l+256, ... in order, then a halving tree
+// over the lanes.  Histograms and marks were updated by other blocks' atomics (in
+// the tail launch, in this kernel): read past L1.
 // The fields of QueryParams the scores use, held in registers.
 struct ScoreParams
 {
@@ -971,7 +971,7 @@ __device__ __forceinline__ void score_finish(const ScoreParams& p, QueryState& s
 #pragma unroll
                     for(int k = 0; k < U; ++k) acc = acc + scored(v[k]);
                 }
-            // (the rest in batches too: read one by one, 16^3 regions took 3 us longer)
+            // (the rest in batches too: read one by one, 16^3 regions took 2.6 us longer)
             constexpr int W = 16;
             for(; r < p.regions; r += W * kScoreLanes)
                 {

@@ -589,10 +589,10 @@ __global__ void __launch_bounds__(kAppendThreads, 8) k_append(const QueryParams*
     // after every tile is done)
     const BaseCache cbase = cache_bases(tile_c_base, n_slots, s_cbase);
     const BaseCache cold = cache_bases(tile_c_old, n_slots - 1, s_cold);
-    // the schedule and tile bases above come from the append kernel before
-    // the propagate kernel this one follows (complete before that propagate
-    // kernel let this one start); the propagate kernel's own results are
-    // read only from here on
+    // the schedule and tile bases above come from the append kernel of the
+    // iteration before (complete before this iteration's propagate kernel, and
+    // through it the score kernels, let this one start); this iteration's
+    // results are read only from here on
     pdl_wait();
     pdl_trigger();
     // First tile static, then tickets, taken only when the block is free: a

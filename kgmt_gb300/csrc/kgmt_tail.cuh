@@ -31,7 +31,7 @@
 // launches that can see each other's words (the host numbers the launches), so
 // the words need no reset.  Every wait is bounded (kErrBarrierTimeout, reported
 // as KGMT_ERR_TIMEOUT).  The launch stops before an iteration that is too large
-// and leaves the state exactly as the two-kernel chain expects it (it recomputes
+// and leaves the state exactly as the chain of launches expects it (it recomputes
 // the schedule), so the host can go on with that chain.
 //
 // Bound by latency: the slowest sample's steps, then about ten dependent L2
@@ -39,7 +39,7 @@
 // straight-line and long, instruction fetches: loops are kept rolled and helpers
 // out of line.  Measured an iteration (double integrator, 20,000-node trees):
 // one query 16.5 us (17.4 with four grid-wide barriers and rows through global
-// memory), 16 queries 22.6 (38 in the two-kernel chain, which took over above
+// memory), 16 queries 22.6 (38 in the chain of launches, which took over above
 // four).
 #pragma once
 #include <climits>
@@ -796,7 +796,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
         }
     if(threadIdx.x == 0) flush();
 
-    // ---- hand the state back: the two-kernel chain's schedule of what is left ----
+    // ---- hand the state back: the chain's schedule of what is left ----
     if(b == 0)
         {
             if(threadIdx.x == 0)
