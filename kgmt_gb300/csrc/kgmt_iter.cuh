@@ -919,12 +919,12 @@ __device__ void update_scores(const ScoreParams& p, QueryState& st, float* lanes
 // Slice `slice` of a larger table: its raw scores into the table, the
 // iteration's new cells into the marks.  Four consecutive regions a thread and
 // round, their counters in 16-byte loads (the tables start 256-byte aligned).
-template <int NT>
+template <int NT, uint32_t SLICE>
 __device__ __forceinline__ void score_slice(const ScoreParams& p, uint32_t slice)
 {
     const float F = (float)p.fine_cells;
-    const uint32_t end = min(p.regions, (slice + 1u) * kScoreSlice);
-    for(uint32_t r = slice * kScoreSlice + threadIdx.x * 4u; r < end; r += NT * 4u)
+    const uint32_t end = min(p.regions, (slice + 1u) * SLICE);
+    for(uint32_t r = slice * SLICE + threadIdx.x * 4u; r < end; r += NT * 4u)
         {
             if(r + 3 < end)
                 {

@@ -504,11 +504,15 @@ __global__ void __launch_bounds__(NT, (MODELS == kBitDI ? 1024 : 512) / NT) k_pr
 // small table whole, or sums and normalises a large one.  Bound by L2 and DRAM
 // latency.  As one launch in which the block that finished a query's last slice
 // summed it, 190 queries of up to 32^3 regions took 75 us (some blocks summed
-// three of them), now 27 + 19.  (Small tables scored by the propagate block that
-// finished the query held that block's next tile up.)
-constexpr int kScoreThreads = 256;
-constexpr int kScoreBlocksPerSm = 6;
-constexpr int kSumThreads = 512;
+// three of them), now 22 + 16.  (Small tables scored by the propagate block that
+// finished the query held that block's next tile up.)  The blocks per SM leave
+// the registers that neither kernel spills: k_score with 256 threads, 6 blocks
+// (40 registers) 28 us, 5 blocks 22, 8 blocks 29; with 128 threads and slices of
+// 512, 6 / 8 / 10 blocks 22.8 / 21.5 / 23.1.  k_score_sum with 512 threads, 2
+// blocks 18.0 us, 1 block 18.9; 256 threads, 2 / 3 blocks 16.9 / 18.4.
+constexpr int kScoreThreads = 128;
+constexpr int kScoreBlocksPerSm = 8;
+constexpr int kSumThreads = 384;
 constexpr int kSumBlocksPerSm = 2;
 
 // whether slot i has a large table to score in this iteration (the schedule's
@@ -542,7 +546,7 @@ __global__ void __launch_bounds__(kScoreThreads, kScoreBlocksPerSm) k_score(cons
             for(uint32_t j = (blockIdx.x + gridDim.x - before % gridDim.x) % gridDim.x; j < total; j += gridDim.x)
                 {
                     const int g = find_slot(s_pre, kScoreThreads, j);
-                    score_slice<kScoreThreads>(score_params(P[c0 + (uint32_t)g]), j - s_pre[g]);
+                    score_slice<kScoreThreads, kScoreSlice>(score_params(P[c0 + (uint32_t)g]), j - s_pre[g]);
                 }
             before += total;
             __syncthreads();

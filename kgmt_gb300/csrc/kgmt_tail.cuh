@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
             Q.epsilon = gp.epsilon, Q.seed = gp.seed;
             Q.node_r1 = gp.node_r1, Q.rep_old = gp.rep_old;
             Q.sp = score_params(gp);
-            Q.slices = Q.sp.regions > kScoreSmall ? (Q.sp.regions + kScoreSlice - 1) / kScoreSlice : 0u;
+            Q.slices = Q.sp.regions > kScoreSmall ? (Q.sp.regions + kTailSlice - 1) / kTailSlice : 0u;
         }
     __syncthreads();
 
@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                     for(int q = 0; q < nq; ++q)
                         if(tq[q].status == KGMT_QUERY_RUNNING && tq[q].slices)
                             {
-                                for(uint32_t j = (b + G - before % G) % G; j < tq[q].slices; j += G) score_slice<NT>(tq[q].sp, j);
+                                for(uint32_t j = (b + G - before % G) % G; j < tq[q].slices; j += G) score_slice<NT, kTailSlice>(tq[q].sp, j);
                                 before += tq[q].slices;
                             }
                     if(!meet(ts, target, acc_block, s_pay, &sched->error)) return;  // (the same payload: it is read below)

@@ -16,13 +16,14 @@ namespace kgmt {
 constexpr int kMaxSampleDim = KGMT_MAX_SAMPLE_DIM;
 constexpr int kScoreLanes = 256;        // fixed summation shape of the score total
 // Region tables of more than kScoreSmall regions are scored by many blocks,
-// kScoreSlice regions each (k_score; the tail launch's scores), smaller ones by
-// one (k_score_sum; the tail launch).  One block took 52 us an iteration for
+// kScoreSlice regions each (k_score; kTailSlice in the tail launch), smaller ones
+// by one (k_score_sum; the tail launch).  One block took 52 us an iteration for
 // 32^3 regions and 6 for 16^3 (three divisions a region on one SM), 1.5 for 8^3.
 // A quadrotor plan in the tail launch, 200 iterations over 16^3 regions: 6.41 ms
 // with the table scored by one block, 6.18 in slices, their meeting included.
 constexpr uint32_t kScoreSmall = 1024;
-constexpr uint32_t kScoreSlice = 1024;
+constexpr uint32_t kScoreSlice = 512;
+constexpr uint32_t kTailSlice = 1024;  // in the tail launch: one round of its blocks' threads
 constexpr int kTileC = 1024;            // samples per append tile
 constexpr int kAppendThreads = 256;     // threads per append block
 constexpr int kAppendPer = kTileC / kAppendThreads;  // samples per append thread
