@@ -62,3 +62,19 @@ def test_order_of_models(n, monkeypatch):
     for i, q in enumerate(qs):
         q.config = q.config.replace(tree_capacity=300 + 40 * (i % 9), max_iterations=3 + i % 4, coarse_len=4, fine_len=2)
     check(qs, monkeypatch)
+
+
+@pytest.mark.parametrize("boxes", [33, 64, 65, 200, 256])
+def test_box_tests_repeat(boxes):
+    """The boxes of a grid cell are listed in order, so the tests made before a
+    first hit, and their sum, are the same for every planner of a scene."""
+    from kgmt_gb300.planner import BatchPlanner
+    qs = W.double_integrator_batch(3, n_obstacles=boxes, seed=7, tree_capacity=6_000, max_iterations=25)
+    counts = set()
+    for _ in range(6):
+        b = BatchPlanner(len(qs))
+        b.plan([q.config for q in qs], *W.pack_queries(qs))
+        st = b.stats()
+        counts.add((st["samples"], st["steps_executed"], st["obstacle_tests"]))
+        b.close()
+    assert len(counts) == 1, counts
