@@ -429,8 +429,21 @@ __global__ void __launch_bounds__(256) k_begin(const __grid_constant__ QueryPara
     compute_schedule(a.params, a.states, a.sched, a.tile_a_base, a.tile_c_base, a.tile_c_old);
 }
 
+// Blocks per SM the registers are shared out for: 24 warps (80 registers) for the
+// models with short steps, 16 (128) where the quadrotor may be met.  256
+// double-integrator / Dubins / unicycle queries in blocks of 256: 3 blocks an SM
+// 2.69 / 2.76 / 0.455 ms of propagate launches, 4 (64 registers, some spilled) 2.76 /
+// 2.77 / 0.474, 2 - / 3.00 / 0.494; in blocks of 512 the double integrator takes
+// two (one: 3.47 against 2.87).
 template <int NT, int MODELS>
-__global__ void __launch_bounds__(NT, (MODELS == kBitDI ? 1024 : 512) / NT) k_propagate(const QueryParams* __restrict__ P, QueryState* S, Sched* sched,
+constexpr int propagate_blocks()
+{
+    if(NT == 512) return MODELS == kBitDI ? 2 : 1;
+    return (MODELS == kBitDI || MODELS == kBitDubins || MODELS == kBitUnicycle ? 768 : 512) / NT;
+}
+
+template <int NT, int MODELS>
+__global__ void __launch_bounds__(NT, propagate_blocks<NT, MODELS>()) k_propagate(const QueryParams* __restrict__ P, QueryState* S, Sched* sched,
                                                   const uint32_t* __restrict__ tile_base, uint32_t smem_boxes)
 {
     // dynamic shared memory of each of the two buffers: grid starts | grid

@@ -94,11 +94,9 @@ constexpr uint32_t kMaxGridItems = 65535;   // grid starts are 16-bit
 // then the boxes -- as many as the launch's box capacity, a power of two
 // from kSmemBoxesMin to kSmemObstacles sized to the admitted queries (what
 // shared memory the boxes leave unused stays L1 cache).  k_propagate has it
-// twice, four blocks an SM.  Propagate launches of 64 double-integrator queries,
-// with 2048 / 3072 / 3584 / 4096 items: of 50 boxes 0.98 / 0.98 / 0.98 / 1.09 ms
-// (too little L1 is left), of 200 boxes 1.19 / 1.14 / 1.14 / 1.13, of 3000 2.26 /
-// 2.23 / 2.09 / 2.08.
-constexpr uint32_t kSmemGridItems = 3584;
+// twice.  Propagate launches of 64 double-integrator queries with 2048 / 3072 /
+// 4096 items: of 200 boxes 1.19 / 1.14 / 1.13 ms, of 3000 2.26 / 2.23 / 2.08.
+constexpr uint32_t kSmemGridItems = 4096;
 constexpr uint32_t kSmemStartBytes = ((kGridCells + 1) * 2 + 15) / 16 * 16;
 constexpr uint32_t kSmemBoxesMin = 64;
 constexpr uint32_t kSmemGridBytes = kSmemStartBytes + kSmemGridItems * 2 + 16;
