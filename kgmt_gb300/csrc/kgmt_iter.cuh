@@ -606,7 +606,8 @@ __device__ __forceinline__ void finish_sample(const QueryParams& p, const GridVi
 // block waited for its longest run and for the sort (2.6 - 2.9 of the 7 - 9
 // warps a scheduler had were at a barrier): iterations of the mixed batch with
 // few samples issued 40 - 48 % of the time, now 63 %; 256 double-integrator
-// queries took 3.12 ms, now 2.81; the 2M-node quadrotor tree 4.63, now 4.25.
+// queries took 3.12 ms, then 2.81 (2.69 with three blocks an SM); the 2M-node
+// quadrotor tree 4.63, then 4.25.
 // ---------------------------------------------------------------------------
 template <int NT>
 struct TileBuf {
