@@ -83,20 +83,32 @@ __device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t* p)
 // block's writes and its word (one fence), adds the block's arrival and waits for
 // all of them (an acquiring read, so every thread's after the barrier); then
 // every thread reads one block's word.  The arrivals only
-// grow: a launch starts from what the last one left.  False when the wait gave up.
-__device__ __noinline__ bool meet(TailScratch* ts, uint32_t& target, uint32_t payload, unsigned long long* pay, uint32_t* error)
+// grow: a launch starts from what the last one left.  The words are kept twice,
+// used by turns: a block that is through may leave its word for the next meeting
+// while a slower one still reads this meeting's (after the goal meeting nothing
+// else holds it back), but it cannot get to the one after, which has this
+// meeting's words, before every block has arrived at the next and so has read
+// them.  False when the wait gave up.
+struct Meeting {
+    uint32_t target;  // arrivals that complete the last meeting
+    uint32_t row;     // words of the next one
+};
+
+__device__ __noinline__ bool meet(TailScratch* ts, Meeting& m, uint32_t payload, unsigned long long* pay, uint32_t* error)
 {
     __shared__ int s_ok;
     __syncthreads();
-    target += gridDim.x;
+    m.target += gridDim.x;
+    uint32_t* word = ts->word[m.row];
+    m.row ^= 1u;
     if(threadIdx.x == 0)
         {
-            *(volatile uint32_t*)&ts->word[blockIdx.x] = payload;
+            *(volatile uint32_t*)&word[blockIdx.x] = payload;
             __threadfence();
             atomicAdd(&ts->arrivals, 1u);
             int ok = 1;
             uint32_t spins = 0;
-            while((int32_t)(ld_acquire_u32(&ts->arrivals) - target) < 0)
+            while((int32_t)(ld_acquire_u32(&ts->arrivals) - m.target) < 0)
                 {
                     if(++spins > kSpinLimit)
                         {
@@ -109,7 +121,7 @@ __device__ __noinline__ bool meet(TailScratch* ts, uint32_t& target, uint32_t pa
             s_ok = ok;
         }
     __syncthreads();
-    if(threadIdx.x < gridDim.x) pay[threadIdx.x] = ld_relaxed_u32(&ts->word[threadIdx.x]);
+    if(threadIdx.x < gridDim.x) pay[threadIdx.x] = ld_relaxed_u32(&word[threadIdx.x]);
     __syncthreads();
     return s_ok != 0;
 }
@@ -376,7 +388,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
     __syncthreads();
 
     uint32_t iters = 0, declined = 0, tag = tag0;
-    uint32_t target = __ldcg(&ts->arrived);  // (rewritten by block 0 after every block's last meeting)
+    Meeting next{__ldcg(&ts->arrived), 0u};  // (arrived is rewritten by block 0 after every block's last meeting)
     int cur_slot = -1;
     uint32_t phase = 0;
     // thread 0: work of the current slot's samples, added to its state when the
@@ -544,7 +556,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
             __syncthreads();
             const uint32_t acc_block = s_sh.acc;
             if(threadIdx.x == 0 && lo < hi) run_steps += s_sh.steps, run_tests += s_sh.tests, run_samples += hi - lo;
-            if(!meet(ts, target, acc_block, s_pay, &sched->error)) return;
+            if(!meet(ts, next, acc_block, s_pay, &sched->error)) return;
 
             // ---- region scores, first of all: every re-activation waits for them ----
             uint32_t large = 0;
@@ -564,7 +576,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                                 for(uint32_t j = (b + G - before % G) % G; j < tq[q].slices; j += G) score_slice<NT, kTailSlice>(tq[q].sp, j);
                                 before += tq[q].slices;
                             }
-                    if(!meet(ts, target, acc_block, s_pay, &sched->error)) return;  // (the same payload: it is read below)
+                    if(!meet(ts, next, acc_block, s_pay, &sched->error)) return;  // (the same payload: it is read below)
                     if(score_q >= 0 && tq[score_q].slices) score_finish<NT>(tq[score_q].sp, S[tq[score_q].slot], s_lanes);
                 }
             if(score_q >= 0)
@@ -734,7 +746,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                         }
                 }
             __syncthreads();
-            if(!meet(ts, target, s_goal_min, s_pay, &sched->error)) return;
+            if(!meet(ts, next, s_goal_min, s_pay, &sched->error)) return;
 
             // ---- finalise (KGMT.cu:88-95, 380-403); every block computes the
             // same state, block 0 writes it back ----
@@ -803,7 +815,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                 {
                     ts->iterations = iters;
                     ts->declined = declined;
-                    ts->arrived = target;
+                    ts->arrived = next.target;
                     atomicAdd(&sched->iterations, iters);
                     if(host_words)
                         {

@@ -256,7 +256,7 @@ struct TailScratch {
     unsigned long long samples;   // samples the tail propagated (host-zeroed)
     uint32_t arrivals;    // blocks' arrivals at meeting points, ever growing
     uint32_t arrived;     // what they were when the last launch ended
-    uint32_t word[kTailMaxBlocks];                // payload of each block's last arrival
+    uint32_t word[2][kTailMaxBlocks];             // payload of each block's arrival, for meetings by turns
     TailBox box[kTailMaxBlocks][kTailMaxBlocks];  // [to][from]
     uint32_t scored[kTailQueries];               // iteration tag: the query's region scores are ready
 };

@@ -1,0 +1,67 @@
+"""The words that the blocks of the tail launch leave for one another, checked on
+the CPU over every order in which a few blocks can get on, with the sizes the
+kernel is compiled with."""
+import functools
+import subprocess
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+
+
+@functools.lru_cache(None)
+def compiled(expr: str) -> str:
+    """An expression over the device descriptors, evaluated by a host program."""
+    import tempfile
+    from kgmt_gb300.build import nvcc
+    include = Path(nvcc()).resolve().parent.parent / "include"
+    with tempfile.TemporaryDirectory() as d:
+        src, exe = Path(d) / "t.cpp", Path(d) / "t"
+        src.write_text(f'#include <cuda_runtime.h>\n#include <iostream>\n#include <type_traits>\n#include "kgmt_types.h"\n'
+                       f"using namespace kgmt;\nint main() {{ std::cout << ({expr}); }}\n")
+        subprocess.run(["g++", "-std=c++17", f"-I{include}", f"-I{ROOT / 'kgmt_gb300' / 'csrc'}", str(src), "-o", str(exe)], check=True)
+        return subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout
+
+
+def stale_reads(blocks: int, meetings: int, rows: int) -> set:
+    """(meeting, meeting whose word was read) of every read that is not of the
+    reader's own meeting.  A block writes its word, arrives, waits for all
+    arrivals, reads every word, and goes on; meeting m uses row m % rows."""
+    start = tuple((0, 0) for _ in range(blocks)), tuple((-1,) * blocks for _ in range(rows))
+    todo, seen, bad = [start], {start}, set()
+    while todo:
+        at, words = todo.pop()
+        for b, (m, step) in enumerate(at):
+            if m == meetings:
+                continue
+            new_words = words
+            if step == 0:  # write
+                row = list(words[m % rows])
+                row[b] = m
+                new_words = words[:m % rows] + (tuple(row),) + words[m % rows + 1:]
+            elif step == 1:  # arrive: counted below by how far each block is
+                pass
+            elif step == 2:  # wait
+                if any((mm, ss) < (m, 2) for mm, ss in at):
+                    continue
+            else:
+                got = words[m % rows][step - 3]
+                if got != m:
+                    bad.add((m, got))
+            nxt = (m, step + 1) if step < 2 + blocks else (m + 1, 0)
+            s = at[:b] + (nxt,) + at[b + 1:], new_words
+            if s not in seen:
+                seen.add(s)
+                todo.append(s)
+    return bad
+
+
+@pytest.mark.parametrize("blocks", [2, 3])
+def test_meeting_words_are_read_before_they_are_written_again(blocks):
+    rows = int(compiled("sizeof(TailScratch::word) / (sizeof(uint32_t) * kTailMaxBlocks)"))
+    assert stale_reads(blocks, 3, rows) == set()
+
+
+def test_one_row_of_words_would_not_do():
+    assert (0, 1) in stale_reads(2, 2, 1)
