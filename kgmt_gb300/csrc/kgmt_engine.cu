@@ -57,6 +57,18 @@ static cudaError_t device_alloc(void** p, size_t bytes)
     return cudaMalloc(p, bytes);
 }
 
+// Polls before a wait of the tail launch gives up.  KGMT_FAULT_TAIL_POLLS=n in
+// the environment (read once) lowers it, for the tests of what follows.
+static uint32_t tail_polls()
+{
+    static const uint32_t polls = [] {
+        const char* e = std::getenv("KGMT_FAULT_TAIL_POLLS");
+        const long n = e ? std::atol(e) : 0;
+        return n > 0 && n < (long)kSpinLimit ? (uint32_t)n : kSpinLimit;
+    }();
+    return polls;
+}
+
 bool is_device_pointer(const void* p)
 {
     cudaPointerAttributes a;
@@ -731,7 +743,8 @@ kgmt_status Engine::run_tail(bool* done, bool* declined_at_once)
     volatile uint32_t* w = h_running_;
     w[2] = 0xFFFFFFFFu;  // a launch that gives up at a meeting point leaves it
     // tags of 2^17 iterations a launch: more than max_iterations allows
-    KGMT_CUDA(launch_tail(args(), d_tail_, models_, tail_grid_[models_], smem_boxes_, tail_max_samples_, tail_seq_ << 17, d_running_ + 2, stream_),
+    KGMT_CUDA(launch_tail(args(), d_tail_, models_, tail_grid_[models_], smem_boxes_, tail_max_samples_, tail_seq_ << 17, tail_polls(), d_running_ + 2,
+                          stream_),
               "k_tail");
     if(profile_)
         {
@@ -748,9 +761,17 @@ kgmt_status Engine::run_tail(bool* done, bool* declined_at_once)
     // a launch that stopped at once left no tags behind
     if(w[2] != 0u) ++tail_seq_;
     KGMT_CUDA(e, "cudaStreamSynchronize");
-    if(w[2] != 0xFFFFFFFFu) tail_iters_ += w[2];
-    // its arrivals are unknown: the next launch starts from none
-    else KGMT_CUDA(cudaMemsetAsync(&d_tail_->arrivals, 0, 2 * sizeof(uint32_t), stream_), "memset(tail)");
+    if(w[2] == 0xFFFFFFFFu)
+        {
+            // It gave up: its arrivals are unknown (the next launch starts from
+            // none), its iteration is half done and the schedule is still the
+            // one from before it, with other sample counts than the states have.
+            // The chain must not run from there.
+            KGMT_CUDA(cudaMemsetAsync(&d_tail_->arrivals, 0, 2 * sizeof(uint32_t), stream_), "memset(tail)");
+            set_error("plan: a device-side wait gave up (tail launch)");
+            return KGMT_ERR_TIMEOUT;
+        }
+    tail_iters_ += w[2];
     *done = w[0] == 0u;
     results_ready_ = *done;
     *declined_at_once = w[3] != 0u && w[2] == 0u;

@@ -1314,7 +1314,7 @@ int tail_blocks_per_sm(int models)
 
 template <int MODELS>
 static cudaError_t launch_tail_t(const LaunchArgs& a, TailScratch* ts, int grid, uint32_t boxes, uint32_t max_samples, uint32_t tag0,
-                                 uint32_t* host_words, cudaStream_t s)
+                                 uint32_t limit, uint32_t* host_words, cudaStream_t s)
 {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -1327,21 +1327,21 @@ static cudaError_t launch_tail_t(const LaunchArgs& a, TailScratch* ts, int grid,
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k_tail<MODELS>, a.params, a.states, a.sched, ts, a.tile_a_base, a.tile_c_base, a.tile_c_old, boxes,
-                              max_samples, tag0, host_words);
+                              max_samples, tag0, limit, host_words);
 }
 
 cudaError_t launch_tail(const LaunchArgs& a, TailScratch* ts, int models, int grid, uint32_t smem_boxes, uint32_t max_samples, uint32_t tag0,
-                        uint32_t* host_words, cudaStream_t s)
+                        uint32_t limit, uint32_t* host_words, cudaStream_t s)
 {
     if(grid < 2 * kTailQueries || grid > kTailMaxBlocks) return cudaErrorInvalidValue;
     const uint32_t boxes = smem_boxes < kSmemBoxesMin ? kSmemBoxesMin : smem_boxes > (uint32_t)kSmemObstacles ? (uint32_t)kSmemObstacles : smem_boxes;
     switch(models)
         {
-            case kBitDI: return launch_tail_t<kBitDI>(a, ts, grid, boxes, max_samples, tag0, host_words, s);
-            case kBitQuad: return launch_tail_t<kBitQuad>(a, ts, grid, boxes, max_samples, tag0, host_words, s);
-            case kBitDubins: return launch_tail_t<kBitDubins>(a, ts, grid, boxes, max_samples, tag0, host_words, s);
-            case kBitUnicycle: return launch_tail_t<kBitUnicycle>(a, ts, grid, boxes, max_samples, tag0, host_words, s);
-            default: return launch_tail_t<kAllModels>(a, ts, grid, boxes, max_samples, tag0, host_words, s);
+            case kBitDI: return launch_tail_t<kBitDI>(a, ts, grid, boxes, max_samples, tag0, limit, host_words, s);
+            case kBitQuad: return launch_tail_t<kBitQuad>(a, ts, grid, boxes, max_samples, tag0, limit, host_words, s);
+            case kBitDubins: return launch_tail_t<kBitDubins>(a, ts, grid, boxes, max_samples, tag0, limit, host_words, s);
+            case kBitUnicycle: return launch_tail_t<kBitUnicycle>(a, ts, grid, boxes, max_samples, tag0, limit, host_words, s);
+            default: return launch_tail_t<kAllModels>(a, ts, grid, boxes, max_samples, tag0, limit, host_words, s);
         }
 }
 

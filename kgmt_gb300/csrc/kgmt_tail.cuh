@@ -30,7 +30,8 @@
 // sums need arrive with the barrier itself.  Tags are never used twice by
 // launches that can see each other's words (the host numbers the launches), so
 // the words need no reset.  Every wait is bounded (kErrBarrierTimeout, reported
-// as KGMT_ERR_TIMEOUT).  The launch stops before an iteration that is too large
+// as KGMT_ERR_TIMEOUT: a launch that gives up leaves the iteration half done, and
+// nothing may go on from its state).  The launch stops before an iteration that is too large
 // and leaves the state exactly as the chain of launches expects it (it recomputes
 // the schedule), so the host can go on with that chain.
 //
@@ -94,7 +95,7 @@ struct Meeting {
     uint32_t row;     // words of the next one
 };
 
-__device__ __noinline__ bool meet(TailScratch* ts, Meeting& m, uint32_t payload, unsigned long long* pay, uint32_t* error)
+__device__ __noinline__ bool meet(TailScratch* ts, Meeting& m, uint32_t payload, unsigned long long* pay, uint32_t limit, uint32_t* error)
 {
     __shared__ int s_ok;
     __syncthreads();
@@ -110,7 +111,7 @@ __device__ __noinline__ bool meet(TailScratch* ts, Meeting& m, uint32_t payload,
             uint32_t spins = 0;
             while((int32_t)(ld_acquire_u32(&ts->arrivals) - m.target) < 0)
                 {
-                    if(++spins > kSpinLimit)
+                    if(++spins > limit)
                         {
                             atomicOr(error, kErrBarrierTimeout);
                             ok = 0;
@@ -134,7 +135,7 @@ __device__ __noinline__ bool meet(TailScratch* ts, Meeting& m, uint32_t payload,
 constexpr int kExchangeBits = 36;
 
 __device__ __noinline__ bool exchange(TailBox (*boxes)[kTailMaxBlocks], unsigned long long payload, uint32_t tag, unsigned long long* pay,
-                                      uint32_t* error)
+                                      uint32_t limit, uint32_t* error)
 {
     __shared__ int s_ok;
     __shared__ unsigned long long s_mine;
@@ -152,7 +153,7 @@ __device__ __noinline__ bool exchange(TailBox (*boxes)[kTailMaxBlocks], unsigned
             uint32_t spins = 0;
             unsigned long long w;
             while(((w = ld_relaxed_u64(from)) >> kExchangeBits) != want)
-                if(++spins > kSpinLimit)
+                if(++spins > limit)
                     {
                         atomicOr(error, kErrBarrierTimeout);
                         s_ok = 0;
@@ -303,7 +304,7 @@ __device__ __forceinline__ uint32_t reactivated32(const TailQuery& Q, uint32_t i
 template <int MODELS>
 __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __restrict__ P, QueryState* S, Sched* sched, TailScratch* ts,
                                                          uint32_t* tile_a_base, uint32_t* tile_c_base, uint32_t* tile_c_old,
-                                                         uint32_t smem_boxes, uint32_t max_samples, uint32_t tag0, uint32_t* host_words)
+                                                         uint32_t smem_boxes, uint32_t max_samples, uint32_t tag0, uint32_t limit, uint32_t* host_words)
 {
     constexpr int NT = kTailThreads;
     constexpr uint32_t kNone = 0xFFFFFFFFu;
@@ -556,7 +557,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
             __syncthreads();
             const uint32_t acc_block = s_sh.acc;
             if(threadIdx.x == 0 && lo < hi) run_steps += s_sh.steps, run_tests += s_sh.tests, run_samples += hi - lo;
-            if(!meet(ts, next, acc_block, s_pay, &sched->error)) return;
+            if(!meet(ts, next, acc_block, s_pay, limit, &sched->error)) return;
 
             // ---- region scores, first of all: every re-activation waits for them ----
             uint32_t large = 0;
@@ -576,7 +577,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                                 for(uint32_t j = (b + G - before % G) % G; j < tq[q].slices; j += G) score_slice<NT, kTailSlice>(tq[q].sp, j);
                                 before += tq[q].slices;
                             }
-                    if(!meet(ts, next, acc_block, s_pay, &sched->error)) return;  // (the same payload: it is read below)
+                    if(!meet(ts, next, acc_block, s_pay, limit, &sched->error)) return;  // (the same payload: it is read below)
                     if(score_q >= 0 && tq[score_q].slices) score_finish<NT>(tq[score_q].sp, S[tq[score_q].slot], s_lanes);
                 }
             if(score_q >= 0)
@@ -667,7 +668,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                         {
                             uint32_t spins = 0;
                             while(ld_relaxed_u32(&ts->scored[qn]) != tag)
-                                if(++spins > kSpinLimit)
+                                if(++spins > limit)
                                     {
                                         atomicOr(&sched->error, kErrBarrierTimeout);
                                         break;
@@ -702,7 +703,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
             }();
             static_assert(2 * kTailAhead <= kTailBitWords, "the nodes drawn ahead use the bits' memory");
             const uint32_t w_block = own & 0x3FFFu;
-            if(!exchange(ts->box, ((unsigned long long)old_block << 14) | w_block, tag, s_pay, &sched->error)) return;
+            if(!exchange(ts->box, ((unsigned long long)old_block << 14) | w_block, tag, s_pay, limit, &sched->error)) return;
 
             // ---- the next frontier's lists ----
             const uint32_t old_before = qn >= 0 ? range_sums(s_pay, tq[qn].node0, b, 14).y : 0u;
@@ -746,7 +747,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                         }
                 }
             __syncthreads();
-            if(!meet(ts, next, s_goal_min, s_pay, &sched->error)) return;
+            if(!meet(ts, next, s_goal_min, s_pay, limit, &sched->error)) return;
 
             // ---- finalise (KGMT.cu:88-95, 380-403); every block computes the
             // same state, block 0 writes it back ----
