@@ -617,6 +617,7 @@ struct TileBuf {
     int q;
     uint32_t first, n;           // samples [first, first + n) of the query
     uint32_t next_run, left;     // runs handed out; warps that are done with the tile
+    uint32_t units;              // kSpinLimit polls each: a wait for the buffer's next tile lasts a run of this one
     PropShared sh;
     uint32_t hist[kSortBins];
     uint16_t rank[kPropPer * NT];  // while sorting: step-count bin and rank in it
@@ -656,6 +657,7 @@ __device__ __forceinline__ void prepare_tile(TileBuf<NT>& B, char* dyn, const Qu
             B.first = lt * tile;
             B.n = min(tile, ns - lt * tile);
             B.next_run = 0, B.left = 0;
+            B.units = wait_units(gp.max_steps, gp.n_obstacles);
             B.sh.acc = 0, B.sh.steps = 0, B.sh.tests = 0;
             // boxes, grid meta, grid starts and the first grid items: one
             // mbarrier transaction of bulk copies (possibly of no bytes)

@@ -476,6 +476,7 @@ __global__ void __launch_bounds__(NT, propagate_blocks<NT, MODELS>()) k_propagat
             mbar_init(&s_buf[0].bar, 1);
             mbar_init(&s_buf[1].bar, 1);
             s_ready[0] = 0, s_ready[1] = 0;
+            s_buf[1].units = 1;
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
     const BaseCache bases = cache_bases(tile_base, n_slots, s_base);
@@ -515,14 +516,21 @@ __global__ void __launch_bounds__(NT, propagate_blocks<NT, MODELS>()) k_propagat
             uint32_t r = 0;
             if(lane == 0)
                 {
-                    uint32_t spins = 0;
+                    // what keeps the tile is the last warp in the buffer's tile
+                    // before, with one run of it at most (its units are still
+                    // there, or those of the tile that is now being prepared)
+                    uint32_t spins = 0, units = *(volatile uint32_t*)&B.units;
                     while((r = s_ready[i & 1u]) != i + 1u && r != kEnd)
                         {
                             if(++spins > kSpinLimit)
                                 {
-                                    atomicOr(&sched->error, kErrCopyTimeout);
-                                    r = kEnd;
-                                    break;
+                                    spins = 0;
+                                    if(--units == 0u)
+                                        {
+                                            atomicOr(&sched->error, kErrCopyTimeout);
+                                            r = kEnd;
+                                            break;
+                                        }
                                 }
                             __nanosleep(20);
                         }

@@ -52,6 +52,18 @@ constexpr int kSparseValidLimit = 10;   // KGMT.cu:336
 constexpr int kSmemObstacles = 512;     // boxes staged in shared memory per block
 constexpr uint32_t kSpinLimit = 1u << 22;  // polls before a device-side wait gives up
 
+// Waits for threads that propagate samples: the time waited for is up to max_steps
+// steps of every box, which the caller sizes (10,000 steps and 65,535 boxes no grid
+// holds are minutes), so the limit grows with it: kSpinLimit polls for each 2^15
+// box tests begun.  A poll takes 18 ns or more, so that is over 2 us a test, and the
+// slowest measured, boxes in global memory, take 0.1.
+__host__ __device__ constexpr uint32_t wait_units(uint32_t max_steps, uint32_t n_obstacles)
+{
+    // 64: the step itself, in box tests
+    const unsigned long long units = 1ull + (max_steps * (n_obstacles + 64ull) >> 15);
+    return units < 0xFFFFFFFFull ? (uint32_t)units : 0xFFFFFFFFu;
+}
+
 constexpr uint32_t kSlotEmpty = 0xFFFFFFFFu;  // QueryState::status of a never-admitted slot
 
 // persistent tail launch (kgmt_tail.cuh): at most this many running queries
