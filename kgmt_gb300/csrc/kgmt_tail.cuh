@@ -89,13 +89,14 @@ __device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t* p)
 // while a slower one still reads this meeting's (after the goal meeting nothing
 // else holds it back), but it cannot get to the one after, which has this
 // meeting's words, before every block has arrived at the next and so has read
-// them.  False when the wait gave up.
+// them.  False when the wait gave up, after limit x units polls.
 struct Meeting {
     uint32_t target;  // arrivals that complete the last meeting
     uint32_t row;     // words of the next one
 };
 
-__device__ __noinline__ bool meet(TailScratch* ts, Meeting& m, uint32_t payload, unsigned long long* pay, uint32_t limit, uint32_t* error)
+__device__ __noinline__ bool meet(TailScratch* ts, Meeting& m, uint32_t payload, unsigned long long* pay, uint32_t limit, uint32_t units,
+                                  uint32_t* error)
 {
     __shared__ int s_ok;
     __syncthreads();
@@ -113,9 +114,13 @@ __device__ __noinline__ bool meet(TailScratch* ts, Meeting& m, uint32_t payload,
                 {
                     if(++spins > limit)
                         {
-                            atomicOr(error, kErrBarrierTimeout);
-                            ok = 0;
-                            break;
+                            spins = 0;
+                            if(--units == 0u)
+                                {
+                                    atomicOr(error, kErrBarrierTimeout);
+                                    ok = 0;
+                                    break;
+                                }
                         }
                     __nanosleep(32);
                 }
@@ -213,6 +218,7 @@ struct TailQuery {
     uint32_t status, itr, tree, n_react, w_new, spe, n_samples, drawn;
     uint32_t slices;  // of a large region table (0: scored by one block)
     uint32_t n_next;  // accepted samples of this iteration
+    uint32_t units;   // of the wait for a sample
     float fa;
     // of the query's params
     uint32_t capacity, samples_per_node, max_iterations;
@@ -325,6 +331,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
     __shared__ unsigned long long s_pay[kTailMaxBlocks];
     __shared__ uint32_t s_goal[kTailQueries], s_goal_min;
     __shared__ int s_score_q, s_qs, s_qn, s_nr, s_too_large;
+    __shared__ uint32_t s_units;
     // the block's samples of this iteration: accepted end rows (dynamic, behind
     // the boxes), parents, and region words with the accept flag
     float* s_rows = (float*)((char*)s_dyn + staged_bytes(smem_boxes));
@@ -384,6 +391,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
             Q.epsilon = gp.epsilon, Q.seed = gp.seed;
             Q.node_r1 = gp.node_r1, Q.rep_old = gp.rep_old;
             Q.sp = score_params(gp);
+            Q.units = wait_units(gp.max_steps, gp.n_obstacles);
             Q.slices = Q.sp.regions > kScoreSmall ? (Q.sp.regions + kTailSlice - 1) / kTailSlice : 0u;
         }
     __syncthreads();
@@ -429,6 +437,9 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                     const uint32_t first = warp_prefix(nb);
                     const unsigned at = __ballot_sync(full, b - first < nb);
                     const unsigned big = __ballot_sync(full, share > kTailShare);
+                    // a block's samples take as many rounds of its threads
+                    constexpr uint32_t kRounds = (kTailShare + NT - 1) / NT;
+                    const uint32_t units = kRounds * min(__reduce_max_sync(full, run ? tq[lane].units : 1u), 0xFFFFFFFFu / kRounds);
                     const uint32_t order = (uint32_t)__popc(running & ((1u << lane) - 1u));
                     // a query's scores are finished by the order-th block from the end
                     const unsigned mine = __ballot_sync(full, run && order == G - 1u - b);
@@ -449,6 +460,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                                     s_score_q = mine ? __ffs((int)mine) - 1 : -1;
                                     s_sh.acc = 0, s_sh.steps = 0, s_sh.tests = 0;
                                     s_goal_min = kNone;
+                                    s_units = units;
                                 }
                             else s_qn = here;
                         }
@@ -557,7 +569,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
             __syncthreads();
             const uint32_t acc_block = s_sh.acc;
             if(threadIdx.x == 0 && lo < hi) run_steps += s_sh.steps, run_tests += s_sh.tests, run_samples += hi - lo;
-            if(!meet(ts, next, acc_block, s_pay, limit, &sched->error)) return;
+            if(!meet(ts, next, acc_block, s_pay, limit, s_units, &sched->error)) return;
 
             // ---- region scores, first of all: every re-activation waits for them ----
             uint32_t large = 0;
@@ -577,7 +589,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                                 for(uint32_t j = (b + G - before % G) % G; j < tq[q].slices; j += G) score_slice<NT, kTailSlice>(tq[q].sp, j);
                                 before += tq[q].slices;
                             }
-                    if(!meet(ts, next, acc_block, s_pay, limit, &sched->error)) return;  // (the same payload: it is read below)
+                    if(!meet(ts, next, acc_block, s_pay, limit, 1u, &sched->error)) return;  // (the same payload: it is read below)
                     if(score_q >= 0 && tq[score_q].slices) score_finish<NT>(tq[score_q].sp, S[tq[score_q].slot], s_lanes);
                 }
             if(score_q >= 0)
@@ -747,7 +759,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                         }
                 }
             __syncthreads();
-            if(!meet(ts, next, s_goal_min, s_pay, limit, &sched->error)) return;
+            if(!meet(ts, next, s_goal_min, s_pay, limit, 1u, &sched->error)) return;
 
             // ---- finalise (KGMT.cu:88-95, 380-403); every block computes the
             // same state, block 0 writes it back ----

@@ -50,3 +50,25 @@ def test_tiles_wait_for_a_long_run(monkeypatch):
     got = plan(q, refused)
     assert got[0]["samples_drawn"] > 200_000
     same(got, plan(q, q.obstacles))
+
+
+@pytest.mark.parametrize("n", [1, 6])
+def test_blocks_meet_after_a_long_run(n):
+    """The blocks of the tail launch wait for the one that has the longest run,
+    some seconds."""
+    from kgmt_gb300.planner import BatchPlanner
+    qs = [query(20_000, 20_000, 1, spn=max(64, 1024 // n), seed=5 + i) for i in range(n)]
+    out = []
+    for k in (0, 1):
+        b = BatchPlanner(n)
+        for q, refused in qs:
+            q.boxes = refused if k else q.obstacles
+        off = np.cumsum([0] + [len(q.boxes) for q, _ in qs])
+        inits, goals, _, _, _ = W.pack_queries([q for q, _ in qs])
+        res = b.plan([q.config for q, _ in qs], inits, goals, np.concatenate([q.boxes for q, _ in qs]), off[:-1], np.diff(off))
+        assert b.stats()["iterations_tail"] == 1
+        out.append([({x: r[x] for x in ("status", "iterations", "tree_size", "goal_index", "samples_drawn")},
+                     tuple(a[: r["tree_size"]] for a in b.copy_tree(i))) for i, r in enumerate(res)])
+        b.close()
+    for a, r in zip(*out):
+        same(a, r)
