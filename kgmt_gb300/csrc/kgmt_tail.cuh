@@ -646,6 +646,9 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
             static_assert(kTailShare * kRepeatSparse < (1u << 14) && kTailShare < (1u << 18), "a block's repeats and rows share one word");
             uint32_t own;
             const uint32_t ex = tail_scan((ca << 14) | cw, s_turn, 0, &own);
+            // the rows appended are the samples counted as accepted, from which every
+            // block has its first row (the chain's finaliser compares them too)
+            if(threadIdx.x == 0 && (own >> 14) != acc_block) atomicOr(&sched->error, kErrAppendMismatch);
             const uint32_t first = qs >= 0 ? tq[qs].tree + acc_before + (ex >> 14) : 0u;
             if(ca)
                 {

@@ -65,3 +65,16 @@ def test_meeting_words_are_read_before_they_are_written_again(blocks):
 
 def test_one_row_of_words_would_not_do():
     assert (0, 1) in stale_reads(2, 2, 1)
+
+
+def test_appended_rows_are_compared_with_the_accepted_samples():
+    """Two counts of the same samples, made apart (one before the rows are placed,
+    one while they are), in the tail launch as in the chain's finaliser: a
+    difference is reported.  Nothing a caller passes makes them differ, so that
+    each compares them is read from the source."""
+    csrc = ROOT / "kgmt_gb300" / "csrc"
+    for name, start in (("kgmt_iter.cuh", "void finalize_query("), ("kgmt_tail.cuh", "k_tail(const QueryParams*")):
+        body = (csrc / name).read_text().split(start, 1)[1]
+        body = body[:body.index("\n}\n")]
+        line = [l for l in body.splitlines() if "kErrAppendMismatch" in l]
+        assert len(line) == 1 and "!=" in line[0] and "atomicOr(&sched->error" in line[0], name
