@@ -192,7 +192,7 @@ class Engine {
     const float* h_paths_ = nullptr;        // the paths' rows in that block
     HostSink sink_ = {};                    // device addresses of the two
     bool results_ready_ = false;  // the last run's states and paths are on the host
-    uint32_t tail_seq_ = 1;       // numbers the tail launches that ran iterations (their tags)
+    unsigned long long tail_seq_ = 1;  // numbers the tail launches that ran iterations (their tags)
     uint32_t* d_running_ = nullptr;  // its device address
     cudaEvent_t ev_[2] = {nullptr, nullptr};
     cudaGraphExec_t graph_ = nullptr;

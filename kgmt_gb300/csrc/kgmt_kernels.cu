@@ -1321,7 +1321,7 @@ int tail_blocks_per_sm(int models)
 }
 
 template <int MODELS>
-static cudaError_t launch_tail_t(const LaunchArgs& a, TailScratch* ts, int grid, uint32_t boxes, uint32_t max_samples, uint32_t tag0,
+static cudaError_t launch_tail_t(const LaunchArgs& a, TailScratch* ts, int grid, uint32_t boxes, uint32_t max_samples, unsigned long long tag0,
                                  uint32_t limit, uint32_t* host_words, cudaStream_t s)
 {
     cudaLaunchAttribute attr[1];
@@ -1338,7 +1338,7 @@ static cudaError_t launch_tail_t(const LaunchArgs& a, TailScratch* ts, int grid,
                               max_samples, tag0, limit, host_words);
 }
 
-cudaError_t launch_tail(const LaunchArgs& a, TailScratch* ts, int models, int grid, uint32_t smem_boxes, uint32_t max_samples, uint32_t tag0,
+cudaError_t launch_tail(const LaunchArgs& a, TailScratch* ts, int models, int grid, uint32_t smem_boxes, uint32_t max_samples, unsigned long long tag0,
                         uint32_t limit, uint32_t* host_words, cudaStream_t s)
 {
     if(grid < 2 * kTailQueries || grid > kTailMaxBlocks) return cudaErrorInvalidValue;

@@ -54,7 +54,7 @@ int tail_blocks_per_sm(int models);
 // tag0: the launch's meeting points are tagged tag0 + 1, ..., one an iteration;
 // no launch since the last one that ran an iteration may have used them.  limit:
 // polls before a wait for the other blocks gives up
-cudaError_t launch_tail(const LaunchArgs& a, TailScratch* ts, int models, int grid, uint32_t smem_boxes, uint32_t max_samples, uint32_t tag0,
+cudaError_t launch_tail(const LaunchArgs& a, TailScratch* ts, int models, int grid, uint32_t smem_boxes, uint32_t max_samples, unsigned long long tag0,
                         uint32_t limit, uint32_t* host_words, cudaStream_t s);
 
 }  // namespace kgmt

@@ -27,9 +27,12 @@
 //
 // A meeting point is an exchange: each block writes one word -- the iteration's
 // tag and a payload -- and reads every block's, so the counts that the prefix
-// sums need arrive with the barrier itself.  Tags are never used twice by
-// launches that can see each other's words (the host numbers the launches), so
-// the words need no reset.  Every wait is bounded (kErrBarrierTimeout, reported
+// sums need arrive with the barrier itself.  The words need no reset: the host
+// numbers the launches, and a tag is the launch's number and the iteration, 64 bits
+// that no engine uses twice.  The mailboxes have room for 28 of them, which come
+// round after 2048 launches; they may, because every iteration rewrites every
+// mailbox, so what a launch finds there is of the launch before it.  The score
+// flags are rewritten only by launches with as many queries, and hold whole tags.  Every wait is bounded (kErrBarrierTimeout, reported
 // as KGMT_ERR_TIMEOUT: a launch that gives up leaves the iteration half done, and
 // nothing may go on from its state).  The launch stops before an iteration that is too large
 // and leaves the state exactly as the chain of launches expects it (it recomputes
@@ -139,12 +142,12 @@ __device__ __noinline__ bool meet(TailScratch* ts, Meeting& m, uint32_t payload,
 // words took 5 us; a mailbox row is read by one block only.)
 constexpr int kExchangeBits = 36;
 
-__device__ __noinline__ bool exchange(TailBox (*boxes)[kTailMaxBlocks], unsigned long long payload, uint32_t tag, unsigned long long* pay,
+__device__ __noinline__ bool exchange(TailBox (*boxes)[kTailMaxBlocks], unsigned long long payload, unsigned long long tag, unsigned long long* pay,
                                       uint32_t limit, uint32_t* error)
 {
     __shared__ int s_ok;
     __shared__ unsigned long long s_mine;
-    const unsigned long long want = ((unsigned long long)tag << kExchangeBits) >> kExchangeBits;  // the tag's bits that fit beside the payload
+    const unsigned long long want = (tag << kExchangeBits) >> kExchangeBits;  // the tag's bits that fit beside the payload
     if(threadIdx.x == 0)
         {
             s_ok = 1;
@@ -310,7 +313,8 @@ __device__ __forceinline__ uint32_t reactivated32(const TailQuery& Q, uint32_t i
 template <int MODELS>
 __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __restrict__ P, QueryState* S, Sched* sched, TailScratch* ts,
                                                          uint32_t* tile_a_base, uint32_t* tile_c_base, uint32_t* tile_c_old,
-                                                         uint32_t smem_boxes, uint32_t max_samples, uint32_t tag0, uint32_t limit, uint32_t* host_words)
+                                                         uint32_t smem_boxes, uint32_t max_samples, unsigned long long tag0, uint32_t limit,
+                                                         uint32_t* host_words)
 {
     constexpr int NT = kTailThreads;
     constexpr uint32_t kNone = 0xFFFFFFFFu;
@@ -396,7 +400,8 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
         }
     __syncthreads();
 
-    uint32_t iters = 0, declined = 0, tag = tag0;
+    uint32_t iters = 0, declined = 0;
+    unsigned long long tag = tag0;
     Meeting next{__ldcg(&ts->arrived), 0u};  // (arrived is rewritten by block 0 after every block's last meeting)
     int cur_slot = -1;
     uint32_t phase = 0;
@@ -598,7 +603,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                     if(threadIdx.x == 0)
                         {
                             __threadfence();
-                            *(volatile uint32_t*)&ts->scored[score_q] = tag;
+                            st_volatile_u64(&ts->scored[score_q], tag);
                         }
                 }
 
@@ -682,13 +687,13 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                     if(threadIdx.x == 0)
                         {
                             uint32_t spins = 0;
-                            while(ld_relaxed_u32(&ts->scored[qn]) != tag)
+                            while(ld_relaxed_u64(&ts->scored[qn]) != tag)
                                 if(++spins > limit)
                                     {
                                         atomicOr(&sched->error, kErrBarrierTimeout);
                                         break;
                                     }
-                            (void)ld_acquire_u32(&ts->scored[qn]);
+                            (void)ld_acquire_u64(&ts->scored[qn]);
                         }
                     __syncthreads();
                     const TailQuery& Q = tq[qn];

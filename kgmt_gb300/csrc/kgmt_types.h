@@ -270,7 +270,7 @@ struct TailScratch {
     uint32_t arrived;     // what they were when the last launch ended
     uint32_t word[2][kTailMaxBlocks];             // payload of each block's arrival, for meetings by turns
     TailBox box[kTailMaxBlocks][kTailMaxBlocks];  // [to][from]
-    uint32_t scored[kTailQueries];               // iteration tag: the query's region scores are ready
+    unsigned long long scored[kTailQueries];      // iteration tag: the query's region scores are ready
 };
 
 }  // namespace kgmt

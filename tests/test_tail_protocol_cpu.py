@@ -78,3 +78,12 @@ def test_appended_rows_are_compared_with_the_accepted_samples():
         body = body[:body.index("\n}\n")]
         line = [l for l in body.splitlines() if "kErrAppendMismatch" in l]
         assert len(line) == 1 and "!=" in line[0] and "atomicOr(&sched->error" in line[0], name
+
+
+def test_score_flags_hold_whole_tags():
+    """A flag may be left from any earlier launch of the engine, so the tag of an
+    iteration (launch number << 17, plus the iteration) must not come round: 2^40
+    launches are thousands of years of planning."""
+    flag = "std::remove_reference_t<decltype(TailScratch::scored[0])>"
+    for launches in (1, 1 << 11, 1 << 15, 1 << 40):
+        assert compiled(f"({flag}(({launches}ull + 7) << 17)) != ({flag}(7ull << 17))") == "1", launches
