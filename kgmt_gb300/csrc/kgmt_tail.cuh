@@ -135,13 +135,11 @@ __device__ __noinline__ bool meet(TailScratch* ts, Meeting& m, uint32_t payload,
     return s_ok != 0;
 }
 
-// The blocks exchange payloads of 36 bits and nothing else: no fence, and no
+// The blocks exchange payloads of kExchangeBits and nothing else: no fence, and no
 // writes ordered by it.  Every block leaves a word with the meeting's tag in
 // every block's own row of mailboxes and waits until its own row has it
 // throughout: one store and one load on the path.  (All blocks polling one row of
 // words took 5 us; a mailbox row is read by one block only.)
-constexpr int kExchangeBits = 36;
-
 __device__ __noinline__ bool exchange(TailBox (*boxes)[kTailMaxBlocks], unsigned long long payload, unsigned long long tag, unsigned long long* pay,
                                       uint32_t limit, uint32_t* error)
 {
@@ -334,7 +332,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
     __shared__ TailQuery tq[kTailQueries];
     __shared__ unsigned long long s_pay[kTailMaxBlocks];
     __shared__ uint32_t s_goal[kTailQueries], s_goal_min;
-    __shared__ int s_score_q, s_qs, s_qn, s_nr, s_too_large;
+    __shared__ int s_score_q, s_qs, s_qn, s_nr, s_too_large, s_too_many;
     __shared__ uint32_t s_units;
     // the block's samples of this iteration: accepted end rows (dynamic, behind
     // the boxes), parents, and region words with the accept flag
@@ -441,7 +439,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                     share = warp == 0 ? (share + 31u) & ~31u : (share + 3u) & ~3u;
                     const uint32_t first = warp_prefix(nb);
                     const unsigned at = __ballot_sync(full, b - first < nb);
-                    const unsigned big = __ballot_sync(full, share > kTailShare);
+                    const unsigned big = __ballot_sync(full, share > (warp == 0 ? kTailShare : kTailNodes));
                     // a block's samples take as many rounds of its threads
                     constexpr uint32_t kRounds = (kTailShare + NT - 1) / NT;
                     const uint32_t units = kRounds * min(__reduce_max_sync(full, run ? tq[lane].units : 1u), 0xFFFFFFFFu / kRounds);
@@ -467,13 +465,13 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                                     s_goal_min = kNone;
                                     s_units = units;
                                 }
-                            else s_qn = here;
+                            else s_qn = here, s_too_many = big != 0u;
                         }
                     if(warp == 0) s_goal[lane] = kNone;
                 }
             __syncthreads();
             if(s_nr == 0) break;
-            if(s_too_large)
+            if(s_too_large | s_too_many)
                 {
                     declined = 1;
                     break;
@@ -648,13 +646,13 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                                 cw += sparse ? kRepeatSparse : kRepeatDense;
                             }
                 }
-            static_assert(kTailShare * kRepeatSparse < (1u << 14) && kTailShare < (1u << 18), "a block's repeats and rows share one word");
+            static_assert(kTailShare * kRepeatSparse < (1u << kRepeatBits) && kTailShare < (1u << 18), "a block's repeats and rows share one word");
             uint32_t own;
-            const uint32_t ex = tail_scan((ca << 14) | cw, s_turn, 0, &own);
+            const uint32_t ex = tail_scan((ca << kRepeatBits) | cw, s_turn, 0, &own);
             // the rows appended are the samples counted as accepted, from which every
             // block has its first row (the chain's finaliser compares them too)
-            if(threadIdx.x == 0 && (own >> 14) != acc_block) atomicOr(&sched->error, kErrAppendMismatch);
-            const uint32_t first = qs >= 0 ? tq[qs].tree + acc_before + (ex >> 14) : 0u;
+            if(threadIdx.x == 0 && (own >> kRepeatBits) != acc_block) atomicOr(&sched->error, kErrAppendMismatch);
+            const uint32_t first = qs >= 0 ? tq[qs].tree + acc_before + (ex >> kRepeatBits) : 0u;
             if(ca)
                 {
                     [[maybe_unused]] const uint32_t cap = s_p.capacity;
@@ -722,18 +720,18 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
                 return old_block - before - n_old;
             }();
             static_assert(2 * kTailAhead <= kTailBitWords, "the nodes drawn ahead use the bits' memory");
-            const uint32_t w_block = own & 0x3FFFu;
-            if(!exchange(ts->box, ((unsigned long long)old_block << 14) | w_block, tag, s_pay, limit, &sched->error)) return;
+            const uint32_t w_block = own & ((1u << kRepeatBits) - 1u);
+            if(!exchange(ts->box, ((unsigned long long)old_block << kRepeatBits) | w_block, tag, s_pay, limit, &sched->error)) return;
 
             // ---- the next frontier's lists ----
-            const uint32_t old_before = qn >= 0 ? range_sums(s_pay, tq[qn].node0, b, 14).y : 0u;
-            const uint32_t w_before = qs >= 0 ? range_sums(s_pay, tq[qs].sample0, b, 14).x : 0u;
+            const uint32_t old_before = qn >= 0 ? range_sums(s_pay, tq[qn].node0, b, kRepeatBits).y : 0u;
+            const uint32_t w_before = qs >= 0 ? range_sums(s_pay, tq[qs].sample0, b, kRepeatBits).x : 0u;
 #pragma unroll 1
             for(int q = NT / 32 - 1 - (int)warp; q < nq; q += NT / 32)
                 {
                     TailQuery& Q = tq[q];
-                    const uint32_t n = range_sums(s_pay, Q.node0, Q.node0 + Q.nodes_nb, 14).y;
-                    const uint32_t w = range_sums(s_pay, Q.sample0, Q.sample0 + Q.samples_nb, 14).x;
+                    const uint32_t n = range_sums(s_pay, Q.node0, Q.node0 + Q.nodes_nb, kRepeatBits).y;
+                    const uint32_t w = range_sums(s_pay, Q.sample0, Q.sample0 + Q.samples_nb, kRepeatBits).x;
                     if(lane == 0 && Q.status == KGMT_QUERY_RUNNING) Q.n_react = n, Q.w_new = w;
                 }
             if(n_old)
@@ -756,7 +754,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const QueryParams* __r
             if(ca)
                 {
                     const uint32_t cap = s_p.capacity;
-                    uint32_t iw = w_before + (ex & 0x3FFFu), idx = first;
+                    uint32_t iw = w_before + (ex & ((1u << kRepeatBits) - 1u)), idx = first;
                     for(uint32_t i = i0; i < i1; ++i)
                         {
                             if(!(s_word[i] >> 31)) continue;

@@ -75,6 +75,12 @@ constexpr int kTailQueries = 32;
 constexpr int kTailThreads = 256;
 constexpr int kTailMaxBlocks = kTailThreads;  // one exchange word a thread
 constexpr uint32_t kTailShare = 640;
+// a block's word in the exchange: its repeats, its re-activated nodes, and the
+// tag's bits that fit beside them.  An iteration in which a block would have more
+// old nodes than the word can count is left to the chain (32 queries of 17 million
+// nodes; one query's 2^28 are 1.8 million a block).
+constexpr int kRepeatBits = 14, kExchangeBits = 36;
+constexpr uint32_t kTailNodes = (1u << (kExchangeBits - kRepeatBits)) - 1u;
 
 // static FP32 lane-operation counts per RK4 step, from the code in
 // kgmt_device.cuh (a multiply, add, fused multiply-add, divide or compare is

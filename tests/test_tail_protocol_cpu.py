@@ -5,6 +5,7 @@ import functools
 import subprocess
 from pathlib import Path
 
+import numpy as np
 import pytest
 
 ROOT = Path(__file__).resolve().parents[1]
@@ -87,3 +88,28 @@ def test_score_flags_hold_whole_tags():
     flag = "std::remove_reference_t<decltype(TailScratch::scored[0])>"
     for launches in (1, 1 << 11, 1 << 15, 1 << 40):
         assert compiled(f"({flag}(({launches}ull + 7) << 17)) != ({flag}(7ull << 17))") == "1", launches
+
+
+def node_share(trees, blocks=152) -> int:
+    """The old nodes a block takes of the query with the most a block, divided as
+    the launch divides them (float32)."""
+    f = np.float32
+    n = np.array(trees, np.uint64)
+    weight = (n + np.uint64(31)) >> np.uint64(5)
+    if len(n) == 1:
+        nb = np.array([blocks])
+    else:
+        nb = 1 + (f(blocks - len(n)) * f(0.99999) * (weight.astype(f) * (f(1) / f(weight.sum())))).astype(np.int64)
+    share = (n.astype(f) * f(1.00001) * (f(1) / nb.astype(f))).astype(np.int64) + 1
+    return int(((share + 3) & ~3).max())
+
+
+def test_counts_fit_the_exchanged_word():
+    """A block's word has as many bits for its re-activated nodes as an iteration
+    that the launch takes can need: all old nodes of the block (a large epsilon
+    re-activates every node).  Trees that a card holds can have more."""
+    nodes, bits = int(compiled("kTailNodes")), int(compiled("kExchangeBits - kRepeatBits"))
+    assert nodes < 1 << bits
+    assert node_share([1 << 28]) <= nodes < node_share([17_000_000] * 32)
+    body = (ROOT / "kgmt_gb300" / "csrc" / "kgmt_tail.cuh").read_text()
+    assert "share > (warp == 0 ? kTailShare : kTailNodes)" in body and "if(s_too_large | s_too_many)" in body
