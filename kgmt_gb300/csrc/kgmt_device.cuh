@@ -324,6 +324,13 @@ struct BlockGrid {
 
 __device__ __forceinline__ uint32_t grid_item(const BlockGrid& g, uint32_t j) { return g.items[j]; }
 
+// No grid: the compiler leaves the cells' code out.
+struct NoGrid {
+    static constexpr const uint16_t* start = nullptr;
+};
+
+__device__ __forceinline__ uint32_t grid_item(const NoGrid&, uint32_t) { return 0u; }
+
 // Consecutive step boxes of a trajectory share an end point, so the grid cell
 // of each end point is computed once and carried into the next step.  Since
 // grid_cell is monotone, the cell range of a step box [min(a, b), max(a, b)]
@@ -344,7 +351,7 @@ __device__ __forceinline__ StepCells start_cells(const QueryParams& P, float x, 
 // (x, then y, then z); more than kGridMaxVisit cells, or a NaN end point, fall
 // back to testing every box.  sc: cells of a on entry, of b on return.
 // PLANAR: z is ignored (a and b carry z = ws_min, grid cell 0).
-// Grid: GridView or BlockGrid.
+// Grid: GridView, BlockGrid or NoGrid.
 template <bool PLANAR = false, typename Grid>
 __device__ __forceinline__ bool step_free(const QueryParams& P, const Grid& grid, const float4* __restrict__ obs, uint32_t n_obs,
                                           float ax, float ay, float az, float bx, float by, float bz, StepCells& sc, PropCount& cnt)

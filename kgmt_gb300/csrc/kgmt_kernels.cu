@@ -967,10 +967,10 @@ __global__ void k_stage_obstacles(const float* __restrict__ src, float4* dst, ui
 // ---------------------------------------------------------------------------
 // Each block stages the boxes, builds the culling grid over them in its own
 // shared memory where that pays (no workspace, nothing shared between calls)
-// and runs a contiguous share of the samples.  Two forms:
+// and runs a contiguous share of the samples.  Four forms:
 //   one sample a thread, blocks of 128 (four warps load the four schedulers of
-//   an SM evenly): up to 256 samples per resident block, where a call's time is
-//   its slowest sample's;
+//   an SM evenly), where a call's time is its slowest sample's: without the grid
+//   (plain, and wide: more and leaner blocks), or with it (culled);
 //   sorted, blocks of 256: each share is counting-sorted by step count, 1024
 //   samples at a time, and the runs of 32 are taken longest first by whichever
 //   warp is free, so a warp's lanes loop equally long.
@@ -979,7 +979,7 @@ __global__ void k_stage_obstacles(const float* __restrict__ src, float4* dst, ui
 // all models that ran one unsorted sample a thread and tested every box at
 // every step: 2^20 quadrotor samples in 200 boxes 352 us, 1631 before; 200,000
 // Dubins samples in 50 boxes 26 us, 60 before; 1000 double-integrator samples
-// in 10 boxes (latency) 4.4 us, 5.0 before.
+// in 5 boxes (latency) 4.1 us, 4.8 before.
 constexpr uint32_t kSamplesChunk = 1024;  // samples sorted at a time
 // dynamic shared memory of the largest call (boxes; the grid's starts and
 // items); the static arrays stay below the 22 KB left of an SM's 227
@@ -992,21 +992,33 @@ static uint32_t samples_items(uint32_t n_obs)
     return (uint32_t)std::min<size_t>(std::max<size_t>(4096, (size_t)n_obs * 8), std::min<size_t>(room, kMaxGridItems));
 }
 static size_t samples_smem(uint32_t n_obs, uint32_t items) { return (size_t)n_obs * 32 + (items ? kGridBuildBytes + (size_t)items * 2 : 0); }
-constexpr int samples_threads(bool sorted) { return sorted ? 256 : 128; }
-// blocks per SM that the kernel is compiled for.  One sample a thread: no
-// spills before warps (1000 double-integrator samples 4.4 us at 3 blocks, 5.0
-// at 4).  Sorted: the quadrotor keeps its state in 128 registers, the other
-// models trade a few spills for more warps (2^20 double-integrator samples in
-// 20 boxes 66 us at 3 blocks, 76 at 2).
-constexpr int samples_blocks(int model, bool sorted) { return !sorted ? 3 : model == KGMT_MODEL_QUADROTOR ? 2 : 3; }
+enum { kSamplesPlain, kSamplesWide, kSamplesCulled, kSamplesSorted };
+constexpr int samples_threads(int form) { return form == kSamplesSorted ? 256 : 128; }
+// Blocks per SM that the forms are compiled for.  Plain and culled: no spills
+// before warps (1000 double-integrator samples in 5 boxes 4.1 us at 3 blocks, 4.4
+// at 5).  Wide: a wave of 97,280 samples (77,000 double-integrator samples in 5
+// boxes 6.9 us at 5 blocks, 8.5 in two waves of 3, 8.5 sorted, 7.0 by the one
+// kernel for all; Dubins 9.8, 12.4, 12.3, 9.8).  The quadrotor has no wide form:
+// sorted, it keeps its state in 128 registers (77,000 samples 32.5 us, 35.5 at 5
+// blocks).  The other models sorted trade a few spills for more warps (2^20
+// double-integrator samples in 20 boxes 66 us at 3 blocks, 76 at 2).
+constexpr int samples_blocks(int model, int form)
+{
+    const bool quad = model == KGMT_MODEL_QUADROTOR;
+    return form == kSamplesWide ? (quad ? 3 : 5) : form == kSamplesSorted && quad ? 2 : 3;
+}
 
-template <int MODEL, bool SORTED>
-__global__ void __launch_bounds__(samples_threads(SORTED), samples_blocks(MODEL, SORTED))
+template <int MODEL, int FORM>
+__global__ void __launch_bounds__(samples_threads(FORM), samples_blocks(MODEL, FORM))
   k_propagate_samples(const __grid_constant__ QueryParams p, const float* x0, const float* __restrict__ uni, const float* __restrict__ obs_rows,
                       uint32_t n_obs, uint32_t n, uint32_t share, uint32_t grid_items, float* x1, uint8_t* valid, int32_t* r1, int32_t* r2)
 {
     constexpr int D = ModelDims<MODEL>::D, NC = ModelDims<MODEL>::NC;
-    constexpr uint32_t NT = (uint32_t)samples_threads(SORTED);
+    constexpr uint32_t NT = (uint32_t)samples_threads(FORM);
+    constexpr bool SORTED = FORM == kSamplesSorted, GRID = FORM == kSamplesCulled || SORTED;
+    // one run a warp: its rows are on their way while the boxes are staged (not
+    // in the wide form, for the registers)
+    constexpr bool AHEAD = FORM == kSamplesPlain || FORM == kSamplesCulled;
     extern __shared__ float4 s_dyn[];
     float4* s_obs = s_dyn;
     char* s_grid = (char*)(s_dyn + 2 * (size_t)n_obs);
@@ -1025,16 +1037,15 @@ __global__ void __launch_bounds__(samples_threads(SORTED), samples_blocks(MODEL,
 #pragma unroll
         for(int j = 0; j < NC + 1; ++j) u[j] = uni[(size_t)s * 8 + j];
     };
-    // one run a warp: its rows are on their way while the boxes are staged
-    if(!SORTED && b0 + threadIdx.x < b1) load(b0 + threadIdx.x);
+    if(AHEAD && b0 + threadIdx.x < b1) load(b0 + threadIdx.x);
     const int w = MODEL == KGMT_MODEL_UNICYCLE ? 2 : 3;
     for(uint32_t i = threadIdx.x; i < n_obs; i += NT) stage_box(obs_rows + (size_t)i * 2 * w, w, s_obs + 2 * i);
     __syncthreads();
-    BlockGrid grid{nullptr, s_items};
-    if(grid_items)
+    std::conditional_t<GRID, BlockGrid, NoGrid> grid;
+    if constexpr(GRID)
         {
             uint32_t total;
-            grid.start = build_grid(p, s_obs, n_obs, grid_items, s_grid, s_scan, s_items, &total);
+            grid = BlockGrid{grid_items ? build_grid(p, s_obs, n_obs, grid_items, s_grid, s_scan, s_items, &total) : nullptr, s_items};
         }
     const unsigned full = 0xffffffffu;
     float* stage = s_stage + warp * 32 * D;
@@ -1098,7 +1109,7 @@ __global__ void __launch_bounds__(samples_threads(SORTED), samples_blocks(MODEL,
                     if(live)
                         {
                             float b[D];
-                            if(SORTED) load(s);
+                            if(!AHEAD) load(s);
                             PropCount cnt;
                             const bool ok = propagate_model<MODEL>(p, grid, a, u, s_obs, n_obs, b, cnt);
                             valid[s] = ok ? 1 : 0;
@@ -1353,7 +1364,7 @@ cudaError_t launch_tail(const LaunchArgs& a, TailScratch* ts, int models, int gr
         }
 }
 
-template <int MODEL, bool SORTED>
+template <int MODEL, int FORM>
 static cudaError_t launch_samples_t(const QueryParams& p, const float* x0, const float* u, const float* obs, uint32_t n_obs, uint32_t n,
                                     uint32_t share, uint32_t items, float* x1, uint8_t* valid, int32_t* r1, int32_t* r2, cudaStream_t s)
 {
@@ -1362,12 +1373,12 @@ static cudaError_t launch_samples_t(const QueryParams& p, const float* x0, const
         {
             // more than 48 KB with the static arrays (always the same limit,
             // so that calls from several threads agree)
-            const cudaError_t e = cudaFuncSetAttribute(k_propagate_samples<MODEL, SORTED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            const cudaError_t e = cudaFuncSetAttribute(k_propagate_samples<MODEL, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                        (int)kSamplesSmemMax);
             if(e != cudaSuccess) return e;
         }
-    k_propagate_samples<MODEL, SORTED><<<(n + share - 1) / share, samples_threads(SORTED), smem, s>>>(p, x0, u, obs, n_obs, n, share, items, x1,
-                                                                                                     valid, r1, r2);
+    k_propagate_samples<MODEL, FORM><<<(n + share - 1) / share, samples_threads(FORM), smem, s>>>(p, x0, u, obs, n_obs, n, share, items, x1,
+                                                                                                 valid, r1, r2);
     return cudaGetLastError();
 }
 
@@ -1386,6 +1397,23 @@ static cudaError_t current_sms(int* sms)
     return e;
 }
 
+// Whether the blocks build the grid: when the box tests it saves take longer than
+// it does.  A test takes about 18 cycles (15 in the plane), the cell walk as much as
+// 8 tests, and the build 10,000 cycles and 40 a box.  The time is that of the longest
+// run: a few samples are not likely to draw the most steps or to last (n / (n + 8) of
+// the way there), and with more than one warp a scheduler each adds 0.7 of its own.  A scene with more
+// boxes than the grid has room for entries has none.  Without / with the grid: 1000
+// Dubins samples in 40 boxes 8.9 / 12.2 us, 640 boxes 81 / 31; 58,000 in 20 boxes 11.7
+// / 15.3, 40 boxes 16.9 / 16.4; 20,000 quadrotor samples in 20 boxes 24.8 / 27.9, 40
+// boxes 29.6 / 28.3; one sample of the double integrator in 500 boxes, which it meets
+// in its first step, 13 / 24.
+static bool samples_culled(const QueryParams& p, uint32_t n_obs, uint32_t n, int sms)
+{
+    if(n_obs <= 8u || samples_items(n_obs) < n_obs) return false;
+    const double warps = std::max(1.0, n / (128.0 * sms)), steps = p.min_steps + (p.max_steps - p.min_steps) * (n / (n + 8.0));
+    return (1.0 + 0.7 * (warps - 1.0)) * steps * (p.planar ? 15.0 : 18.0) * (n_obs - 8.0) > 10000.0 + 40.0 * n_obs;
+}
+
 template <int MODEL>
 static cudaError_t launch_samples_m(const QueryParams& p, const float* x0, const float* u, const float* obs, uint32_t n_obs, uint32_t n, float* x1,
                                     uint8_t* valid, int32_t* r1, int32_t* r2, cudaStream_t s)
@@ -1393,24 +1421,32 @@ static cudaError_t launch_samples_m(const QueryParams& p, const float* x0, const
     int sms = 0;
     const cudaError_t e = current_sms(&sms);
     if(e != cudaSuccess) return e;
-    // The grid is built when the box tests it saves cost more than it does: a
-    // test is about 12 instructions a step, the cell walk about as much as 10
-    // tests, and the build about 5500 cycles, while the samples take
-    // n / (128 SMs) rounds of one warp per scheduler.  Measured without / with
-    // the grid (before the two forms were split): 8193 Dubins samples in 100
-    // boxes 17.8 / 15.4 us, 30 boxes 9.9 / 12.3; 49,999 in 50 boxes 20.9 /
-    // 17.4, 20 boxes 12.8 / 15.7; 2^20 in 20 boxes 124 / 105.
-    const double rounds = std::max(1.0, n / (128.0 * sms)), steps = 0.5 * (p.min_steps + p.max_steps);
-    const uint32_t items = rounds * steps * 12.0 * ((double)n_obs - 10.0) > 5500.0 ? samples_items(n_obs) : 0u;
-    // sorted shares once the samples fill the resident blocks more than once
-    // (200,000 quadrotor samples in 50 boxes: 73 us sorted, 148 unsorted)
-    const uint32_t per_sm =
-      (uint32_t)std::max<size_t>(1, std::min<size_t>((size_t)samples_blocks(MODEL, true), 227 * 1024 / (samples_smem(n_obs, items) + 22 * 1024)));
-    const uint32_t blocks = (uint32_t)sms * per_sm;
-    if(n <= blocks * (uint32_t)samples_threads(true))
-        return launch_samples_t<MODEL, false>(p, x0, u, obs, n_obs, n, (uint32_t)samples_threads(false), items, x1, valid, r1, r2, s);
+    const uint32_t items = samples_culled(p, n_obs, n, sms) ? samples_items(n_obs) : 0u;
+    const size_t smem = samples_smem(n_obs, items);
+    // blocks that are resident together
+    auto resident = [&](int form) {
+        const size_t each = smem + (size_t)samples_threads(form) * ModelDims<MODEL>::D * 4 + 4096;  // the stage, the small arrays
+        const size_t fit = std::max<size_t>(1, 227 * 1024 / each);
+        return (uint32_t)sms * (uint32_t)std::min<size_t>((size_t)samples_blocks(MODEL, form), fit);
+    };
+    // one sample a thread while the resident blocks have a thread for each, else
+    // sorted shares (200,000 quadrotor samples in 50 boxes: 73 us sorted, 148 not)
+    constexpr uint32_t nt = (uint32_t)samples_threads(kSamplesPlain);
+    if(items)
+        {
+            if(n <= resident(kSamplesCulled) * nt)
+                return launch_samples_t<MODEL, kSamplesCulled>(p, x0, u, obs, n_obs, n, nt, items, x1, valid, r1, r2, s);
+        }
+    else if(n <= resident(kSamplesPlain) * nt)
+        return launch_samples_t<MODEL, kSamplesPlain>(p, x0, u, obs, n_obs, n, nt, 0u, x1, valid, r1, r2, s);
+    else if constexpr(MODEL != KGMT_MODEL_QUADROTOR)
+        {
+            if(n <= resident(kSamplesWide) * nt)
+                return launch_samples_t<MODEL, kSamplesWide>(p, x0, u, obs, n_obs, n, nt, 0u, x1, valid, r1, r2, s);
+        }
+    const uint32_t blocks = resident(kSamplesSorted);
     const uint32_t share = ((n + blocks - 1) / blocks + 31u) & ~31u;
-    return launch_samples_t<MODEL, true>(p, x0, u, obs, n_obs, n, share, items, x1, valid, r1, r2, s);
+    return launch_samples_t<MODEL, kSamplesSorted>(p, x0, u, obs, n_obs, n, share, items, x1, valid, r1, r2, s);
 }
 
 cudaError_t launch_propagate_samples(const QueryParams& p, const float* x0, const float* u, const float* obs, uint32_t n_obs, uint32_t n,

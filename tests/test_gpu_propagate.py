@@ -101,3 +101,17 @@ def test_boxes_the_grid_must_not_lose(kind, n):
         b[:, 3:] = b[:, :3] + 0.012
     x0, u = inputs(q.config, n, 17)
     check(q.config, x0, u, b)
+
+
+@pytest.mark.parametrize("model", sorted(MAKE))
+@pytest.mark.parametrize("n,n_obs", [(58_368, 7), (58_369, 9), (97_280, 9), (97_281, 7), (1, 400), (9, 400), (600, 5_200), (600, 6_000), (20_000, 5_300)])
+def test_edges_of_the_forms(model, n, n_obs):
+    """A full wave of the plain and of the wide form and one sample more, and few
+    samples and very many boxes, where the grid does not pay or has no room."""
+    q = MAKE[model](seed=11, n_obstacles=n_obs if n_obs < 100 else 50)
+    if n_obs >= 100:
+        rng = np.random.default_rng(n_obs)
+        lo = rng.uniform(0.0, 0.97, (n_obs, 3)).astype(np.float32)
+        q.obstacles = np.concatenate([lo, lo + np.float32(0.01)], 1)
+    x0, u = inputs(q.config, n, n + n_obs)
+    check(q.config, x0, u, q.obstacles)
