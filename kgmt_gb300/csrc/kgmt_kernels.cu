@@ -236,9 +236,12 @@ __global__ void k_admit(const QueryParams* __restrict__ P, QueryState* S, uint32
 // ---------------------------------------------------------------------------
 // The cells' 16-bit counters (two a word) become the fill cursors in place,
 // and a filled cell's cursor is the start of the next one: with a zero before
-// the first, they are the CSR starts.  Four lanes share a box, an x slice
-// each: a lane's chain of shared-memory atomics on a box's 8 to 30 cells is
-// the longest part of the build.
+// the first, they are the CSR starts.  While the block has lanes to spare, four
+// or two of them share a box, an x slice each: a lane's chain of shared-memory
+// atomics on a box's 8 to 30 cells is the longest part of a small build.  With more
+// boxes than that a lane a box: boxes are smaller there, and lanes beyond a box's
+// slices idle (four lanes for any number: a plan's first iteration with 10,000 boxes
+// 281 us, now 147; 1000 samples in 2000 boxes 74 and 41).
 constexpr uint32_t kGridBuildBytes = 16 + kGridCells * 2;  // shared memory of a build
 // The grids of batches, which count their box tests, list the boxes of a cell in
 // increasing order when they have at most kGridOrdered of them in at most
@@ -254,12 +257,20 @@ constexpr uint32_t kGridOrderedItems = 8192;
 template <typename F>
 __device__ __forceinline__ bool for_box_cells(const QueryParams& p, const float4* obs, uint32_t n, F&& f)
 {
-    constexpr int SHARE = 4, G = (int)kGridDim;
+    constexpr int G = (int)kGridDim;
+    const uint32_t sh = n * 4u <= blockDim.x ? 2u : n * 2u <= blockDim.x ? 1u : 0u;  // log2 of the lanes a box
+    const uint32_t step = blockDim.x >> sh;
     bool bad = false;
+    // the next box is on its way while this one's cells are counted (64 queries of
+    // 10,000 boxes, admission and an iteration: 432 us without, 411 with)
+    uint32_t o = threadIdx.x >> sh;
+    float4 na = make_float4(0.0f, 0.0f, 0.0f, 0.0f), nb = na;
+    if(o < n) na = obs[2 * o], nb = obs[2 * o + 1];
 #pragma unroll 1
-    for(uint32_t o = threadIdx.x / SHARE; o < n; o += blockDim.x / SHARE)
+    for(; o < n; o += step)
         {
-            const float4 a = obs[2 * o], b = obs[2 * o + 1];
+            const float4 a = na, b = nb;
+            if(o + step < n) na = obs[2 * (o + step)], nb = obs[2 * (o + step) + 1];
             if(isnan(a.x) || isnan(a.y) || isnan(a.z) || isnan(b.x) || isnan(b.y) || isnan(b.z))
                 {
                     bad = true;
@@ -269,7 +280,7 @@ __device__ __forceinline__ bool for_box_cells(const QueryParams& p, const float4
             const int y0 = grid_cell(p, fminf(a.y, b.y)), y1 = grid_cell(p, fmaxf(a.y, b.y));
             const int z0 = p.planar ? 0 : grid_cell(p, fminf(a.z, b.z)), z1 = p.planar ? 0 : grid_cell(p, fmaxf(a.z, b.z));
 #pragma unroll 1
-            for(int cx = x0 + (int)(threadIdx.x % SHARE); cx <= x1; cx += SHARE)
+            for(int cx = x0 + (int)(threadIdx.x & ((1u << sh) - 1u)); cx <= x1; cx += 1 << sh)
 #pragma unroll 1
                 for(int cy = y0; cy <= y1; ++cy)
                     for(int cz = z0; cz <= z1; ++cz) f(o, (cx * G + cy) * G + cz);
@@ -404,8 +415,9 @@ __global__ void __launch_bounds__(256) k_begin(const __grid_constant__ QueryPara
     QueryParams* dst = const_cast<QueryParams*>(a.params);
     for(uint32_t i = threadIdx.x; i < sizeof(QueryParams) / 4; i += blockDim.x) ((uint32_t*)dst)[i] = ((const uint32_t*)&p)[i];
     static_assert(sizeof(QueryParams) % 4 == 0 && sizeof(QueryState) % 8 == 0, "copied by words");
-    for(uint32_t o = threadIdx.x; o < p.n_obstacles; o += blockDim.x)
-        stage_box(p.raw_obstacles + (size_t)o * 2 * p.raw_w, p.raw_w, p.obstacles + 2 * o);
+    if(p.raw_obstacles)  // (else they are staged)
+        for(uint32_t o = threadIdx.x; o < p.n_obstacles; o += blockDim.x)
+            stage_box(p.raw_obstacles + (size_t)o * 2 * p.raw_w, p.raw_w, p.obstacles + 2 * o);
     admit_root(p, a.states[0]);
     if(threadIdx.x == 0)
         {
@@ -1399,7 +1411,7 @@ static cudaError_t current_sms(int* sms)
 
 // Whether the blocks build the grid: when the box tests it saves take longer than
 // it does.  A test takes about 18 cycles (15 in the plane), the cell walk as much as
-// 8 tests, and the build 10,000 cycles and 40 a box.  The time is that of the longest
+// 8 tests, and the build 10,000 cycles and 30 a box.  The time is that of the longest
 // run: a few samples are not likely to draw the most steps or to last (n / (n + 8) of
 // the way there), and with more than one warp a scheduler each adds 0.7 of its own.  A scene with more
 // boxes than the grid has room for entries has none.  Without / with the grid: 1000
@@ -1411,7 +1423,7 @@ static bool samples_culled(const QueryParams& p, uint32_t n_obs, uint32_t n, int
 {
     if(n_obs <= 8u || samples_items(n_obs) < n_obs) return false;
     const double warps = std::max(1.0, n / (128.0 * sms)), steps = p.min_steps + (p.max_steps - p.min_steps) * (n / (n + 8.0));
-    return (1.0 + 0.7 * (warps - 1.0)) * steps * (p.planar ? 15.0 : 18.0) * (n_obs - 8.0) > 10000.0 + 40.0 * n_obs;
+    return (1.0 + 0.7 * (warps - 1.0)) * steps * (p.planar ? 15.0 : 18.0) * (n_obs - 8.0) > 10000.0 + 30.0 * n_obs;
 }
 
 template <int MODEL>
