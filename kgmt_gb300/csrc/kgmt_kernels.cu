@@ -236,12 +236,13 @@ __global__ void k_admit(const QueryParams* __restrict__ P, QueryState* S, uint32
 // ---------------------------------------------------------------------------
 // The cells' 16-bit counters (two a word) become the fill cursors in place,
 // and a filled cell's cursor is the start of the next one: with a zero before
-// the first, they are the CSR starts.  While the block has lanes to spare, four
-// or two of them share a box, an x slice each: a lane's chain of shared-memory
-// atomics on a box's 8 to 30 cells is the longest part of a small build.  With more
-// boxes than that a lane a box: boxes are smaller there, and lanes beyond a box's
-// slices idle (four lanes for any number: a plan's first iteration with 10,000 boxes
-// 281 us, now 147; 1000 samples in 2000 boxes 74 and 41).
+// the first, they are the CSR starts.  Where that takes fewer or shorter rounds,
+// four lanes share a box, an x slice each: a lane's chain of shared-memory atomics
+// on a box's 8 to 30 cells is the longest part of a small build.  More boxes get a
+// lane each: they are smaller, and lanes beyond a box's slices idle.  (1000 Dubins
+// samples, blocks of 128: 100 boxes 14.2 us by four lanes, 13.6 by one; 160 boxes 16.2,
+// 18.7; 256 boxes 20.0, 17.7; 2000 boxes of the double integrator 74, 41.  A plan's first
+// iteration with 10,000 boxes 281, 147.)
 constexpr uint32_t kGridBuildBytes = 16 + kGridCells * 2;  // shared memory of a build
 // The grids of batches, which count their box tests, list the boxes of a cell in
 // increasing order when they have at most kGridOrdered of them in at most
@@ -258,7 +259,8 @@ template <typename F>
 __device__ __forceinline__ bool for_box_cells(const QueryParams& p, const float4* obs, uint32_t n, F&& f)
 {
     constexpr int G = (int)kGridDim;
-    const uint32_t sh = n * 4u <= blockDim.x ? 2u : n * 2u <= blockDim.x ? 1u : 0u;  // log2 of the lanes a box
+    // log2 of the lanes a box: a round of four lanes a box takes 3/8 of one of a lane
+    const uint32_t sh = 3u * ((n * 4u + blockDim.x - 1u) / blockDim.x) < 8u * ((n + blockDim.x - 1u) / blockDim.x) ? 2u : 0u;
     const uint32_t step = blockDim.x >> sh;
     bool bad = false;
     // the next box is on its way while this one's cells are counted (64 queries of
