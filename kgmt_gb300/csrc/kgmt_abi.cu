@@ -205,7 +205,7 @@ static kgmt_status plan_setup(kgmt_planner* p, const float* h_initial, const flo
     p->params.raw_obstacles = n_obstacles ? d_obstacles : nullptr;
     p->params.raw_w = (int32_t)ws_dims_of(p->cfg.model);
     p->eng.set_models(Engine::model_bit(p->cfg.model));
-    p->eng.set_max_obstacles(n_obstacles);
+    p->eng.set_max_obstacles(staged_count(n_obstacles));
     p->eng.set_large_tables(p->params.regions > kScoreSmall);
     const kgmt_status st = p->eng.admit_only(p->params);
     p->params.raw_obstacles = nullptr;  // the caller's array
@@ -436,7 +436,7 @@ static kgmt_status batch_prepare(kgmt_batch* b, uint32_t n, const kgmt_config* c
             total += L[i].total;
             uint64_t end = (uint64_t)obs_offset[i] + obs_count[i];
             if(end > boxes) boxes = end;
-            if(obs_count[i] > max_obs) max_obs = obs_count[i];
+            max_obs = std::max(max_obs, staged_count(obs_count[i]));
             if(cfgs[i].max_iterations > max_iters) max_iters = cfgs[i].max_iterations;
             max_regions = std::max(max_regions, regions_of(cfgs[i]));
         }
@@ -729,7 +729,7 @@ struct kgmt_server {
     std::deque<kgmt_result> done;
     uint64_t next_ticket = 1;
     uint32_t resident = 0;     // admitted and not yet retired
-    uint32_t box_capacity = 0; // boxes a propagate block stages: the largest admitted so far
+    uint32_t box_capacity = 0; // most staged boxes of a query admitted so far
     uint32_t max_regions = 0;  // the largest region table admitted so far
     bool resched = false;      // a resident query was cancelled: the next step recomputes the schedule
     // the step in flight: its iterations and the copy of states [0, copied)
@@ -884,7 +884,7 @@ extern "C" kgmt_status kgmt_server_step(kgmt_server* s, uint32_t* n_running, uin
             r.ticket = q.ticket;
             r.offset = off;
             r.submitted = q.submitted;
-            if(n_obs > s->box_capacity) s->box_capacity = n_obs;
+            s->box_capacity = std::max(s->box_capacity, staged_count(n_obs));
             s->max_regions = std::max(s->max_regions, prm.regions);
             ++s->resident;
             ++slot;

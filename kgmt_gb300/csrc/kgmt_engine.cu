@@ -521,9 +521,9 @@ kgmt_status Engine::set_prop_block(uint32_t block)
     return KGMT_OK;
 }
 
-void Engine::set_max_obstacles(uint32_t max_obs)
+void Engine::set_max_obstacles(uint32_t most)
 {
-    const uint32_t boxes = smem_boxes_for(max_obs);
+    const uint32_t boxes = smem_boxes_for(most);
     if(boxes == smem_boxes_) return;
     smem_boxes_ = boxes;
     if(graph_)
@@ -685,10 +685,10 @@ kgmt_status Engine::record_event(cudaEvent_t* out)
 // variant or the boxes it stages change)
 int Engine::propagate_grid()
 {
-    const uint32_t key = (uint32_t)models_ << 16 | smem_boxes_;
+    const uint32_t boxes = prop_boxes_for(smem_boxes_, prop_block_), key = (uint32_t)models_ << 16 | boxes;
     if(prop_grid_for_ != key)
         {
-            prop_grid_ = sms_ * propagate_blocks_per_sm((int)prop_block_, models_, smem_boxes_);
+            prop_grid_ = sms_ * propagate_blocks_per_sm((int)prop_block_, models_, boxes);
             prop_grid_for_ = key;
         }
     return prop_grid_;
@@ -708,7 +708,8 @@ kgmt_status Engine::launch_iteration()
                 }
             if(k == 0)
                 {
-                    KGMT_CUDA(launch_propagate(a, (int)prop_block_, models_, propagate_grid(), smem_boxes_, stream_), "k_propagate");
+                    KGMT_CUDA(launch_propagate(a, (int)prop_block_, models_, propagate_grid(), prop_boxes_for(smem_boxes_, prop_block_), stream_),
+                              "k_propagate");
                     KGMT_CUDA(launch_score(a, sms_, large_tables_, stream_), "k_score");
                 }
             else KGMT_CUDA(launch_append(a, grid_c_, stream_), "k_append");

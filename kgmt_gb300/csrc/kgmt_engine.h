@@ -126,9 +126,9 @@ class Engine {
     // kernel variant (single-model variants, or the one for any mix); a
     // change drops the graph
     void set_models(int mask);
-    // largest box count of the admitted queries: sizes the propagate kernel's
+    // largest staged_count of the admitted queries: sizes the propagate kernel's
     // shared-memory box stage (a change drops the graph)
-    void set_max_obstacles(uint32_t max_obs);
+    void set_max_obstacles(uint32_t most);
     // whether an admitted query may have more than kScoreSmall regions: the
     // chain then has a k_score launch (a change drops the graph)
     void set_large_tables(bool large);
@@ -176,7 +176,7 @@ class Engine {
     int sms_ = 0;
     bool large_tables_ = true;      // the chain scores large region tables in their own launch
     int models_ = 15;               // propagate variant (Engine::variant_of)
-    uint32_t smem_boxes_ = kSmemObstacles;  // boxes staged in shared memory per propagate block
+    uint32_t smem_boxes_ = kSmemObstacles;  // box capacity of the admitted queries' stages
     QueryParams* d_params_ = nullptr;
     QueryState* d_states_ = nullptr;
     Sched* d_sched_ = nullptr;

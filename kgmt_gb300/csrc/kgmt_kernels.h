@@ -18,9 +18,9 @@ struct LaunchArgs {
 // admits slots [first, first + count), or slots[0 .. count) (device memory) when given
 cudaError_t launch_admit(const LaunchArgs& a, uint32_t first, uint32_t count, cudaStream_t s, const uint32_t* slots = nullptr);
 cudaError_t launch_schedule(const LaunchArgs& a, cudaStream_t s);
-// models: bit 0 double integrator, bit 1 quadrotor (the mix the launch may meet)
-// smem_boxes: boxes a block stages in shared memory (the largest query of the
-// launch, rounded by smem_boxes_for); more are read from global memory
+// models: Engine::model_bit of those the launch may meet
+// smem_boxes: boxes a block has room to stage in shared memory (prop_boxes_for);
+// a query of more is read from global memory
 cudaError_t launch_propagate(const LaunchArgs& a, int block, int models, int grid, uint32_t smem_boxes, cudaStream_t s);
 // region scores, between propagate and append; large: whether some query has
 // more than kScoreSmall regions

@@ -180,7 +180,8 @@ extern "C" kgmt_status kgmt_plan_noalloc(const kgmt_config* cfg, const float* h_
     NA_CHECK(cuda_status(cudaGetDevice(&dev), "cudaGetDevice"));
     NA_CHECK(cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute"));
     const int models = Engine::variant_of(Engine::model_bit(cfg->model));
-    const int grid_a = sms * propagate_blocks_per_sm((int)block, models, smem_boxes_for(n_obstacles));
+    const uint32_t boxes = prop_boxes_for(staged_count(n_obstacles), block);
+    const int grid_a = sms * propagate_blocks_per_sm((int)block, models, boxes);
     const int grid_c = sms * append_blocks_per_sm();
 
     // the array keeps the previous call's contents: reset what starts at zero
@@ -209,7 +210,7 @@ extern "C" kgmt_status kgmt_plan_noalloc(const kgmt_config* cfg, const float* h_
         {
             for(int k = 0; k < 4; ++k)
                 {
-                    NA_CHECK(cuda_status(launch_propagate(a, (int)block, models, grid_a, smem_boxes_for(n_obstacles), s), "k_propagate"));
+                    NA_CHECK(cuda_status(launch_propagate(a, (int)block, models, grid_a, boxes, s), "k_propagate"));
                     NA_CHECK(cuda_status(launch_score(a, sms, params.regions > kScoreSmall, s), "k_score"));
                     NA_CHECK(cuda_status(launch_append(a, grid_c, s), "k_append"));
                 }

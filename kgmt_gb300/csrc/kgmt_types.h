@@ -120,12 +120,25 @@ constexpr uint32_t kSmemBoxesMin = 64;
 constexpr uint32_t kSmemGridBytes = kSmemStartBytes + kSmemGridItems * 2 + 16;
 __host__ __device__ constexpr uint32_t staged_bytes(uint32_t boxes) { return kSmemGridBytes + boxes * 32; }
 __host__ __device__ constexpr uint32_t prop_smem_bytes(uint32_t boxes) { return 2 * staged_bytes(boxes); }
-// box capacity for queries of at most max_obs boxes
-inline uint32_t smem_boxes_for(uint32_t max_obs)
+// what a query of n boxes adds to a launch's box capacity: nothing where its boxes
+// are too many to stage and are read from global memory (a stage for them, twice and
+// unused, left two blocks an SM: 96 Dubins queries of 3000 boxes 8.37 ms, now 7.90)
+inline uint32_t staged_count(uint32_t n) { return n <= (uint32_t)kSmemObstacles ? n : 0u; }
+// box capacity for queries of at most `most` staged boxes
+inline uint32_t smem_boxes_for(uint32_t most)
 {
     uint32_t c = kSmemBoxesMin;
-    while(c < max_obs && c < (uint32_t)kSmemObstacles) c <<= 1;
+    while(c < most && c < (uint32_t)kSmemObstacles) c <<= 1;
     return c;
+}
+// of a propagate launch.  Blocks of 128 with two stages of more than 128 boxes would
+// be two an SM: those boxes stay in global memory (96 Dubins queries of 300 / 512
+// boxes 6.18 / 6.41 ms with one stage a block, 6.69 / 7.12 with two, 6.03 / 6.34 so; of
+// 100 boxes 5.52 staged, 5.56 not).
+inline uint32_t prop_boxes_for(uint32_t most, uint32_t block)
+{
+    const uint32_t c = smem_boxes_for(most);
+    return block == 128u && c > 128u ? kSmemBoxesMin : c;
 }
 
 // error bits in Sched::error

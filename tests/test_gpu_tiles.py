@@ -78,3 +78,14 @@ def test_box_tests_repeat(boxes):
         counts.add((st["samples"], st["steps_executed"], st["obstacle_tests"]))
         b.close()
     assert len(counts) == 1, counts
+
+
+@pytest.mark.parametrize("block", [128, 256, 512])
+@pytest.mark.parametrize("most", [128, 129, 512, 700])
+def test_boxes_staged_and_not_in_one_launch(block, most, monkeypatch):
+    """Queries whose boxes a launch stages beside some whose boxes it leaves in
+    global memory: above 512, and in blocks of 128 above 64 once any has over 128."""
+    qs = W.double_integrator_batch(6, n_obstacles=most, seed=most, tree_capacity=4_000, max_iterations=10)
+    for q, n in zip(qs, (0, 10, 64, 65, most // 2, most)):
+        q.obstacles = q.obstacles[:n]
+    check(qs, monkeypatch, block)
