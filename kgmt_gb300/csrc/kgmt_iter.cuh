@@ -693,15 +693,15 @@ __device__ __forceinline__ void prepare_tile(TileBuf<NT>& B, char* dyn, const Qu
     sync();
     if(!BLOCK || lane < 32u)
         {
-    const uint32_t v = B.hist[lane];
-    uint32_t x = v;
+            const uint32_t v = B.hist[lane];
+            uint32_t x = v;
 #pragma unroll
-    for(int o = 1; o < 32; o <<= 1)
-        {
-            const uint32_t y = __shfl_up_sync(full, x, o);
-            if(lane >= (uint32_t)o) x += y;
-        }
-    B.hist[lane] = x - v;
+            for(int o = 1; o < 32; o <<= 1)
+                {
+                    const uint32_t y = __shfl_up_sync(full, x, o);
+                    if(lane >= (uint32_t)o) x += y;
+                }
+            B.hist[lane] = x - v;
         }
     sync();
     for(uint32_t i = lane; i < n; i += W)
@@ -793,10 +793,13 @@ __device__ __forceinline__ void propagate_range(const QueryParams& sp, const Pro
     });
 }
 
-// Graph::updateVertices (Graph.cu:311-358) for one query: all regions scored,
-// lane l of kScoreLanes sums regions l, l+256, ... in order, then a halving tree
-// over the lanes.  Histograms and marks were updated by other blocks' atomics (in
-// the tail launch, in this kernel): read past L1.
+// ---------------------------------------------------------------------------
+// region scores: Graph::updateVertices (Graph.cu:311-358).  All regions of a query
+// are scored, lane l of kScoreLanes sums regions l, l+256, ... in order, then a
+// halving tree over the lanes; a small table by update_scores, a large one by
+// score_slice and score_finish.  Histograms and marks were updated by other blocks'
+// atomics (in the tail launch, in this kernel): read past L1.
+// ---------------------------------------------------------------------------
 // The fields of QueryParams the scores use, held in registers.
 struct ScoreParams
 {
@@ -865,21 +868,23 @@ __device__ __forceinline__ float lanes_total(float* lanes)
     return lanes[0];
 }
 
-// a table of at most kScoreSmall regions, by one block
+// a table of at most kScoreSmall regions, by one block: a lane a thread
 template <int NT>
 __device__ void update_scores(const ScoreParams& p, QueryState& st, float* lanes)
 {
+    static_assert(NT >= kScoreLanes, "a lane a thread");
     const float F = (float)p.fine_cells;
     constexpr int U = (int)kScoreSmall / kScoreLanes;  // a lane's regions: loaded together, their raw scores kept in registers
+    const uint32_t l = threadIdx.x;
     float kept[U];
-    for(int l = threadIdx.x; l < kScoreLanes; l += NT)
+    if(l < (uint32_t)kScoreLanes)
         {
             uint64_t m[U];
             int32_t nv[U], n[U];
 #pragma unroll
             for(int k = 0; k < U; ++k)
                 {
-                    const uint32_t r = (uint32_t)l + k * kScoreLanes;
+                    const uint32_t r = l + k * kScoreLanes;
                     if(r < p.regions)
                         {
                             m[k] = __ldcg(&p.marks[r]) | __ldcg(&p.newmarks[r]);
@@ -892,29 +897,21 @@ __device__ void update_scores(const ScoreParams& p, QueryState& st, float* lanes
 #pragma unroll
             for(int k = 0; k < U; ++k)
                 {
-                    const uint32_t r = (uint32_t)l + k * kScoreLanes;
+                    const uint32_t r = l + k * kScoreLanes;
                     if(r >= p.regions) break;
                     p.marks[r] = m[k];
                     p.newmarks[r] = 0ull;
-                    const float raw = raw_score(p, F, m[k], nv[k], n[k]);
-                    if(l == (int)threadIdx.x) kept[k] = raw;
-                    else p.score[r] = raw;
-                    acc = acc + scored(raw);
+                    kept[k] = raw_score(p, F, m[k], nv[k], n[k]);
+                    acc = acc + scored(kept[k]);
                 }
             lanes[l] = acc;
         }
     const float total = lanes_total(lanes);
-    for(int l = threadIdx.x; l < kScoreLanes; l += NT)
+    if(l < (uint32_t)kScoreLanes)
         {
-            uint32_t r = (uint32_t)l;
-            if(l == (int)threadIdx.x)
-                {
 #pragma unroll
-                    for(int k = 0; k < U; ++k, r += kScoreLanes)
-                        if(r < p.regions) p.score[r] = norm_score(p, kept[k], total);
-                }
-            // more lanes than threads: the rest re-reads what it wrote itself
-            for(; r < p.regions; r += kScoreLanes) p.score[r] = norm_score(p, p.score[r], total);
+            for(int k = 0; k < U; ++k)
+                if(l + k * kScoreLanes < p.regions) p.score[l + k * kScoreLanes] = norm_score(p, kept[k], total);
         }
     if(threadIdx.x == 0) st.score_total = total;
 }
@@ -1008,9 +1005,6 @@ __device__ __forceinline__ void score_finish(const ScoreParams& p, QueryState& s
     if(threadIdx.x == 0) st.score_total = total;
 }
 
-// MODELS: bit 0 double integrator present, bit 1 quadrotor present; the
-// launch picks the variant for the admitted mix, so a single-model batch
-// pays for one model's registers only
 // ---------------------------------------------------------------------------
 // append / re-activation / frontier build
 // ---------------------------------------------------------------------------

@@ -583,10 +583,7 @@ __global__ void __launch_bounds__(NT, propagate_blocks<NT, MODELS>()) k_propagat
 // summed it, 190 queries of up to 32^3 regions took 75 us (some blocks summed
 // three of them), now 22 + 16.  (Small tables scored by the propagate block that
 // finished the query held that block's next tile up.)  The blocks per SM leave
-// the registers that neither kernel spills: k_score with 256 threads, 6 blocks
-// (40 registers) 28 us, 5 blocks 22, 8 blocks 29; with 128 threads and slices of
-// 512, 6 / 8 / 10 blocks 22.8 / 21.5 / 23.1.  k_score_sum with 512 threads, 2
-// blocks 18.0 us, 1 block 18.9; 256 threads, 2 / 3 blocks 16.9 / 18.4.
+// each kernel the registers it does not spill.
 constexpr int kScoreThreads = 128;
 constexpr int kScoreBlocksPerSm = 8;
 constexpr int kSumThreads = 384;

@@ -112,8 +112,8 @@ constexpr uint32_t kMaxGridItems = 65535;   // grid starts are 16-bit
 // then the boxes -- as many as the launch's box capacity, a power of two
 // from kSmemBoxesMin to kSmemObstacles sized to the admitted queries (what
 // shared memory the boxes leave unused stays L1 cache).  k_propagate has it
-// twice.  Propagate launches of 64 double-integrator queries with 2048 / 3072 /
-// 4096 items: of 200 boxes 1.19 / 1.14 / 1.13 ms, of 3000 2.26 / 2.23 / 2.08.
+// twice.  Fewer items staged would make room for more blocks but were slower (64
+// double-integrator queries of 3000 boxes, 2048 items: 2.26 ms of propagate, 2.08).
 constexpr uint32_t kSmemGridItems = 4096;
 constexpr uint32_t kSmemStartBytes = ((kGridCells + 1) * 2 + 15) / 16 * 16;
 constexpr uint32_t kSmemBoxesMin = 64;
