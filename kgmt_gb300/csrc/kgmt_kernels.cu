@@ -1007,12 +1007,12 @@ enum { kSamplesPlain, kSamplesWide, kSamplesCulled, kSamplesSorted };
 constexpr int samples_threads(int form) { return form == kSamplesSorted ? 256 : 128; }
 // Blocks per SM that the forms are compiled for.  Plain and culled: no spills
 // before warps (1000 double-integrator samples in 5 boxes 4.1 us at 3 blocks, 4.4
-// at 5).  Wide: a wave of 97,280 samples (77,000 double-integrator samples in 5
-// boxes 6.9 us at 5 blocks, 8.5 in two waves of 3, 8.5 sorted, 7.0 by the one
-// kernel for all; Dubins 9.8, 12.4, 12.3, 9.8).  The quadrotor has no wide form:
-// sorted, it keeps its state in 128 registers (77,000 samples 32.5 us, 35.5 at 5
-// blocks).  The other models sorted trade a few spills for more warps (2^20
-// double-integrator samples in 20 boxes 66 us at 3 blocks, 76 at 2).
+// at 5).  Wide: a wave of 97,280 samples (77,000 double-integrator samples in 20
+// boxes 9.5 us at 5 blocks, 10.5 in two waves of 3, 12.0 sorted, 9.7 by the one kernel
+// for all; Dubins 14.9, 15.6, 17.6, 14.7).  The quadrotor has no wide form: sorted, it
+// keeps its state in 128 registers (77,000 samples in 20 boxes 38 us, 42 at 5 blocks).
+// The other models sorted trade a few spills for more warps (2^20 double-integrator
+// samples in 20 boxes 66 us at 3 blocks, 76 at 2).
 constexpr int samples_blocks(int model, int form)
 {
     const bool quad = model == KGMT_MODEL_QUADROTOR;
