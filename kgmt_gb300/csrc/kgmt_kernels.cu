@@ -1410,7 +1410,7 @@ static cudaError_t current_sms(int* sms)
 
 // Whether the blocks build the grid: when the box tests it saves take longer than
 // it does.  A test takes about 18 cycles (15 in the plane), the cell walk as much as
-// 8 tests, and the build 10,000 cycles and 30 a box.  The time is that of the longest
+// 8 tests, and the build 10,500 cycles and 30 a box.  The time is that of the longest
 // run: a few samples are not likely to draw the most steps or to last (n / (n + 8) of
 // the way there), and with more than one warp a scheduler each adds 0.7 of its own.  A scene with more
 // boxes than the grid has room for entries has none.  Without / with the grid: 1000
@@ -1422,7 +1422,7 @@ static bool samples_culled(const QueryParams& p, uint32_t n_obs, uint32_t n, int
 {
     if(n_obs <= 8u || samples_items(n_obs) < n_obs) return false;
     const double warps = std::max(1.0, n / (128.0 * sms)), steps = p.min_steps + (p.max_steps - p.min_steps) * (n / (n + 8.0));
-    return (1.0 + 0.7 * (warps - 1.0)) * steps * (p.planar ? 15.0 : 18.0) * (n_obs - 8.0) > 10000.0 + 30.0 * n_obs;
+    return (1.0 + 0.7 * (warps - 1.0)) * steps * (p.planar ? 15.0 : 18.0) * (n_obs - 8.0) > 10500.0 + 30.0 * n_obs;
 }
 
 template <int MODEL>
