@@ -239,9 +239,9 @@ __global__ void k_admit(const QueryParams* __restrict__ P, QueryState* S, uint32
 // the first, they are the CSR starts.  Where that takes fewer or shorter rounds,
 // four lanes share a box, an x slice each: a lane's chain of shared-memory atomics
 // on a box's 8 to 30 cells is the longest part of a small build.  More boxes get a
-// lane each: they are smaller, and lanes beyond a box's slices idle.  (1000 Dubins
-// samples, blocks of 128: 100 boxes 14.2 us by four lanes, 13.6 by one; 160 boxes 16.2,
-// 18.7; 256 boxes 20.0, 17.7; 2000 boxes of the double integrator 74, 41.  A plan's first
+// lane each: they are smaller, and lanes beyond a box's slices idle.  (49,999 Dubins
+// samples, blocks of 128: 80 boxes 17.2 us by four lanes, 17.6 by one; 100 boxes 18.4,
+// 17.7; 160 boxes 21.0, 23.3; 256 boxes 24.3, 21.8; 640 boxes 37.0, 25.2.  A plan's first
 // iteration with 10,000 boxes 281, 147.)
 constexpr uint32_t kGridBuildBytes = 16 + kGridCells * 2;  // shared memory of a build
 // The grids of batches, which count their box tests, list the boxes of a cell in
@@ -255,24 +255,25 @@ constexpr uint32_t kGridOrderedItems = 8192;
 
 // calls f(o, cell) for the cells of the boxes o, this thread's share of them;
 // true when a box has a NaN coordinate (its cells are skipped)
-template <typename F>
+template <bool GLOBAL, typename F>
 __device__ __forceinline__ bool for_box_cells(const QueryParams& p, const float4* obs, uint32_t n, F&& f)
 {
     constexpr int G = (int)kGridDim;
-    // log2 of the lanes a box: a round of four lanes a box takes 3/8 of one of a lane
-    const uint32_t sh = 3u * ((n * 4u + blockDim.x - 1u) / blockDim.x) < 8u * ((n + blockDim.x - 1u) / blockDim.x) ? 2u : 0u;
+    // log2 of the lanes a box: a round of four lanes a box takes 5/16 of one of a lane
+    const uint32_t sh = 5u * ((n * 4u + blockDim.x - 1u) / blockDim.x) < 16u * ((n + blockDim.x - 1u) / blockDim.x) ? 2u : 0u;
     const uint32_t step = blockDim.x >> sh;
     bool bad = false;
-    // the next box is on its way while this one's cells are counted (64 queries of
-    // 10,000 boxes, admission and an iteration: 432 us without, 411 with)
+    // in global memory the next box is on its way while this one's cells are counted
+    // (64 queries of 10,000 boxes, admission and an iteration: 432 us without, 411 with)
     uint32_t o = threadIdx.x >> sh;
     float4 na = make_float4(0.0f, 0.0f, 0.0f, 0.0f), nb = na;
-    if(o < n) na = obs[2 * o], nb = obs[2 * o + 1];
+    if(GLOBAL && o < n) na = obs[2 * o], nb = obs[2 * o + 1];
 #pragma unroll 1
     for(; o < n; o += step)
         {
+            if(!GLOBAL) na = obs[2 * o], nb = obs[2 * o + 1];
             const float4 a = na, b = nb;
-            if(o + step < n) na = obs[2 * (o + step)], nb = obs[2 * (o + step) + 1];
+            if(GLOBAL && o + step < n) na = obs[2 * (o + step)], nb = obs[2 * (o + step) + 1];
             if(isnan(a.x) || isnan(a.y) || isnan(a.z) || isnan(b.x) || isnan(b.y) || isnan(b.z))
                 {
                     bad = true;
@@ -296,6 +297,8 @@ __device__ __forceinline__ bool for_box_cells(const QueryParams& p, const float4
 // 256) must enter.  Returns the starts (kGridCells + 1 of them, inside mem; starts and
 // items are complete: the build ends with a block barrier), or nullptr when
 // the grid is unusable; *total gets the entries.
+// GLOBAL: the boxes are in global memory (else staged).
+template <bool GLOBAL>
 __device__ __forceinline__ const uint16_t* build_grid(const QueryParams& p, const float4* obs, uint32_t n, uint32_t budget, char* mem,
                                                       uint32_t* scratch, uint16_t* items, uint32_t* total, uint16_t* listed = nullptr)
 {
@@ -306,7 +309,7 @@ __device__ __forceinline__ const uint16_t* build_grid(const QueryParams& p, cons
     if(threadIdx.x == 0) s_bad = n > kMaxObstacles ? 1 : 0;
     __syncthreads();
     const uint32_t boxes = n > kMaxObstacles ? 0u : n;
-    if(for_box_cells(p, obs, boxes, [&](uint32_t, int c) { atomicAdd(&cursor[c >> 1], 1u << ((c & 1) * 16)); })) s_bad = 1;
+    if(for_box_cells<GLOBAL>(p, obs, boxes, [&](uint32_t, int c) { atomicAdd(&cursor[c >> 1], 1u << ((c & 1) * 16)); })) s_bad = 1;
     __syncthreads();
     // counts -> exclusive prefixes; a thread owns 16 (or, of 128, 32)
     // consecutive cells.  Pairs of 16-bit counts are summed in 32 bits.
@@ -334,7 +337,7 @@ __device__ __forceinline__ const uint16_t* build_grid(const QueryParams& p, cons
     __syncthreads();
     const bool ordered = listed && boxes <= kGridOrdered && *total <= kGridOrderedItems;
     uint16_t* const fill = ordered ? listed : items;
-    for_box_cells(p, obs, boxes, [&](uint32_t o, int c) {
+    for_box_cells<GLOBAL>(p, obs, boxes, [&](uint32_t o, int c) {
         const int sh = (c & 1) * 16;
         fill[(atomicAdd(&cursor[c >> 1], 1u << sh) >> sh) & 0xffffu] = (uint16_t)o;
     });
@@ -383,7 +386,7 @@ __global__ void __launch_bounds__(256) k_build_grid(const QueryParams* __restric
     const QueryParams& p = P[slots ? slots[blockIdx.x] : first + blockIdx.x];
     if(p.grid_start == nullptr) return;
     uint32_t total = 0;
-    const uint16_t* start = build_grid(p, p.obstacles, p.n_obstacles, p.grid_budget, mem, scratch, p.grid_items, &total, listed);
+    const uint16_t* start = build_grid<true>(p, p.obstacles, p.n_obstacles, p.grid_budget, mem, scratch, p.grid_items, &total, listed);
     if(start)
         for(uint32_t c = threadIdx.x; c <= kGridCells; c += 256) p.grid_start[c] = start[c];
     if(threadIdx.x == 0)
@@ -431,7 +434,7 @@ __global__ void __launch_bounds__(256) k_begin(const __grid_constant__ QueryPara
     if(p.grid_start != nullptr)
         {
             uint32_t total = 0;
-            const uint16_t* start = build_grid(p, p.obstacles, p.n_obstacles, p.grid_budget, mem, scratch, p.grid_items, &total);
+            const uint16_t* start = build_grid<true>(p, p.obstacles, p.n_obstacles, p.grid_budget, mem, scratch, p.grid_items, &total);
             if(start)
                 for(uint32_t c = threadIdx.x; c <= kGridCells; c += blockDim.x) p.grid_start[c] = start[c];
             if(threadIdx.x == 0)
@@ -1056,7 +1059,7 @@ __global__ void __launch_bounds__(samples_threads(FORM), samples_blocks(MODEL, F
     if constexpr(GRID)
         {
             uint32_t total;
-            grid = BlockGrid{grid_items ? build_grid(p, s_obs, n_obs, grid_items, s_grid, s_scan, s_items, &total) : nullptr, s_items};
+            grid = BlockGrid{grid_items ? build_grid<false>(p, s_obs, n_obs, grid_items, s_grid, s_scan, s_items, &total) : nullptr, s_items};
         }
     const unsigned full = 0xffffffffu;
     float* stage = s_stage + warp * 32 * D;
